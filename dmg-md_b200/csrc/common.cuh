@@ -121,12 +121,25 @@ struct __align__(32) Site {
   long long type;
 };
 
-// A site record as two 16-byte loads: a = (x, y), c = (z, type bits).
+// A site record in one 32-byte load: a = (x, y), c = (z, type bits).  Of 32
+// scattered records in L1 the load pipe takes 26 cycles as two 16-byte loads
+// each, 17.5 as one of 32 bytes, and the sweeps over neighbours are bound by it.
 __device__ __forceinline__ void site_load(const Site* __restrict__ sites, int j, double2& a,
                                           double2& c)
 {
-  a = __ldg(reinterpret_cast<const double2*>(sites + j));
-  c = __ldg(reinterpret_cast<const double2*>(sites + j) + 1);
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(a.x), "=d"(a.y), "=d"(c.x), "=d"(c.y)
+      : "l"(sites + j));
+}
+
+// The same of a record that this launch may have written (coherent load).
+__device__ __forceinline__ void site_load_coherent(const Site* sites, int j, double2& a,
+                                                   double2& c)
+{
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(a.x), "=d"(a.y), "=d"(c.x), "=d"(c.y)
+               : "l"(sites + j)
+               : "memory");
 }
 
 // Displacement from (xi, yi, zi) to a loaded site and the site's type, same
@@ -201,6 +214,31 @@ __device__ __forceinline__ void skin_check_atom(int N, int i, const Box& b, doub
   if ((dx * dx + dy * dy + dz * dz) > half_skin_sq) st->rebuild = 1;
 }
 
+// Two FP32 multiply-adds (or products) in one instruction: sm_100a's packed
+// pairs, each half rounded as fmaf() rounds it.  The moment and force sweeps
+// are bound by the instructions they issue, and half of those were FMAs.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
+{
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
 // Cutoff function fc = (1 + cos(pi d / rc)) / 2 and its d-derivative.
 // FAST (the mixed-precision kernels): sine and cosine from the hardware
 // approximations (absolute error about 4e-7 on [0, pi)) in place of the
@@ -234,6 +272,12 @@ __device__ __forceinline__ void edge_length(float d2, float& d, float& dinv)
   }
 }
 
+// Functions past the model's basis multiply zero coefficients (the tables'
+// rows are zero-padded), so a short basis is evaluated whole, without a
+// comparison per function.
+template <int KMAX>
+__host__ __device__ constexpr bool whole_basis() { return KMAX <= 9; }
+
 // Shifted Chebyshev radial basis f_k(d) = (T_k(x) + 1) / 2 * fc (f_0 = fc)
 // with x = 2 (d/rc - 1)^2 - 1, k = 0..kmax-1.
 template <int KMAX>
@@ -246,7 +290,7 @@ __device__ __forceinline__ void radial_basis(int kmax, float rcinv, float d, flo
   fn[0] = fc;
 #pragma unroll
   for (int k = 1; k < KMAX; ++k) {
-    if (k < kmax) fn[k] = (t1 + 1.0f) * half_fc;
+    if (whole_basis<KMAX>() || k < kmax) fn[k] = (t1 + 1.0f) * half_fc;
     const float t2 = 2.0f * x * t1 - t0;
     t0 = t1;
     t1 = t2;
@@ -267,7 +311,7 @@ __device__ __forceinline__ void radial_basis_d(int kmax, float rcinv, float d, f
   fnp[0] = fcp;
 #pragma unroll
   for (int k = 1; k < KMAX; ++k) {
-    if (k < kmax) {
+    if (whole_basis<KMAX>() || k < kmax) {
       fn[k] = 0.5f * (t1 + 1.0f) * fc;
       fnp[k] = 0.5f * (dt1 * dxdd * fc + (t1 + 1.0f) * fcp);
     }

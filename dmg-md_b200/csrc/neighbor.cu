@@ -427,8 +427,8 @@ k_neighbor_rebuild(const RebuildArgs a)
         const int local = k - (r_incl - r_cnt);
         const int at = local < r_n1 ? r_st1 + local : r_st2 + (local - r_n1);
         j = a.cell_atoms[at];
-        const double2 sa = reinterpret_cast<const double2*>(a.cell_sites + at)[0];
-        const double2 sc = reinterpret_cast<const double2*>(a.cell_sites + at)[1];
+        double2 sa, sc;
+        site_load_coherent(a.cell_sites, at, sa, sc);
         float dx, dy, dz;
         int tj;
         site_delta(b, sa, sc, xi, yi, zi, dx, dy, dz, tj);
