@@ -395,9 +395,16 @@ __host__ __device__ inline int filter_bin_float4(const ModelParams& p, int kp)
   const int q = p.T * kp / 4;
   return q | 1;
 }
-__host__ __device__ inline bool filter_bins(const ModelParams& p, int kp)
+// Where the filter keeps its bins (BIN): nowhere (the contraction per edge),
+// shared memory, or registers: one type and the short basis (10 of them; two
+// types' 20, or the long basis's 18, cost more than they save: water 24k
+// descriptor stage 114 us with shared bins, 123 us with registers).
+constexpr int kBinNone = 0, kBinShared = 1, kBinRegs = 2;
+template <int KM>
+int filter_bin(const ModelParams& p)
 {
-  return p.T * kp <= kFilterBinMax;
+  if (p.T == 1 && KM <= 9) return kBinRegs;
+  return p.T * ((KM + 3) & ~3) <= kFilterBinMax ? kBinShared : kBinNone;
 }
 
 // Neighbour type of an edge record (float4: displacement, type << 28 | index).
@@ -767,21 +774,21 @@ __device__ void tc_ann(const ModelParams& p, const FusedLayout& Lay, float* sm, 
 // expression; nep.cu:503-561) and writes the radial and angular rows in
 // order (group ballot + popcount), summing
 // q_n = sum_j sum_k c(ti,tj)[n][k] f_k(d_ij) on the way.  BIN: each lane
-// sums its edges' basis values per neighbour type, B[tj][k] += f_k(d_ij), in
-// its own shared-memory bins and contracts them with c once at the end
-// (q_n = sum_t sum_k c(ti,t)[n][k] B[t][k]): a few float4 updates per edge
-// instead of the nR x kR contraction.  Kept apart from k_nep_fused so this
+// sums its edges' basis values per neighbour type, B[tj][k] += f_k(d_ij), and
+// contracts them with c once at the end (q_n = sum_t sum_k c(ti,t)[n][k]
+// B[t][k]) instead of the nR x kR contraction per edge.  The bins of one
+// type are registers, those of several the lane's own shared memory (1M
+// carbon, descriptor stage: 3.51 ms with shared bins, 3.48 with registers).
+// Kept apart from k_nep_fused so this
 // latency-bound sweep runs at the occupancy of its own register count.
 // The angular edges are also written out, displacement and neighbour type, to
 // the slots their forces f12 will take: the descriptor kernel then sweeps 16
 // contiguous bytes per edge instead of fetching sites, and overwrites each
-// slot with the force once it has read it (descriptor stage of 1M carbon 4.03 ->
-// 3.76 ms, water 24k 0.142 -> 0.121 ms; its sites came through shared-memory
-// prefetch slots before).
+// slot with the force once it has read it.
 // FAST: the mixed-precision build (hardware sqrt / reciprocal / sine-cosine
 // approximations, see cutoff_fc), held to seven CTAs per SM (72 registers,
 // as the exact build takes; it would take 78, rounded to 80: six CTAs).
-template <int G, int NRM, int KM, bool BIN, bool FAST>
+template <int G, int NRM, int KM, int BIN, bool FAST>
 __global__ void __launch_bounds__(kBlock, (FAST ? 7 : 0))
 k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
                 const Site* __restrict__ sites, NeighborState* st,
@@ -802,7 +809,7 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
   // this lane's bins [T][KP] (an odd number of float4 per lane: no bank conflicts)
   float4* bin = reinterpret_cast<float4*>(sm + filter_table_floats(p, KP)) +
                 tid * filter_bin_float4(p, KP);
-  if constexpr (BIN)
+  if constexpr (BIN == kBinShared)
     for (int q = 0; q < T * KP / 4; ++q) bin[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (blockIdx.x == 0 && tid == 0) st->rebuild = 0;   // the Verlet list is consumed
   __syncthreads();
@@ -818,6 +825,9 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
   float qr[NRM];
 #pragma unroll
   for (int n = 0; n < NRM; ++n) qr[n] = 0.0f;
+  float rb[KP];
+#pragma unroll
+  for (int k = 0; k < KP; ++k) rb[k] = 0.0f;
   const int nv = active ? nn_v[i] : 0;
   const int nv_max = __reduce_max_sync(kFull, nv);
   const int* vrow = nl_v + static_cast<size_t>(i) * mn_v;
@@ -870,7 +880,10 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
 #pragma unroll
       for (int kk = 0; kk < KP; ++kk) fn[kk] = 0.0f;
       radial_basis<KM>(kR, rcinv, d, fc, fn);
-      if constexpr (BIN) {
+      if constexpr (BIN == kBinRegs) {
+#pragma unroll
+        for (int k = 0; k < KM; ++k) rb[k] += fn[k];
+      } else if constexpr (BIN == kBinShared) {
         float4* bt = bin + t2 * (KP / 4);
 #pragma unroll
         for (int q = 0; q < KP / 4; ++q) {
@@ -898,7 +911,11 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
     cr += __popc(mr);
     ca += __popc(ma);
   }
-  if constexpr (BIN) {
+  if constexpr (BIN == kBinRegs) {
+#pragma unroll
+    for (int n = 0; n < NRM; ++n)
+      if (n < nR) qr[n] += dot_basis<KM>(sm + n * KP, rb);
+  } else if constexpr (BIN == kBinShared) {
     const float* bf = reinterpret_cast<const float*>(bin);
     for (int t = 0; t < T; ++t) {
       const float* c = sm + (t1 * T + t) * nR * KP;
@@ -933,15 +950,15 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
 // table for the pair (nA rows of the padded basis, shared memory).
 // Reference find_partial_force_angular (nep.cu:890-991) with the
 // accumulate_f12 ladder (nep_utilities.cuh:1240-1491) evaluated once per edge
-// instead of once per (edge, n).
-template <int KM, int NAM, int LMAX, bool AG = true, bool FAST = false, bool EX = false>
+// instead of once per (edge, n).  (Degrees 5 to 8; angular_edge_force4 below.)
+template <int KM, int NAM, int LMAX, bool AG, bool FAST>
 __device__ __forceinline__ float3 angular_edge_force(const ModelParams& p, const float* c,
                                                     const float* __restrict__ av, float rc,
                                                     float rcinv, float dx, float dy, float dz)
 {
   constexpr int KP = (KM + 3) & ~3;
   constexpr int NLM = num_lm<LMAX>();
-  const int nA = EX ? NAM : p.nA, L_max = EX ? LMAX : p.L_max;
+  const int nA = p.nA, L_max = p.L_max;
   float d, dinv;
   edge_length<FAST>(dx * dx + dy * dy + dz * dz, d, dinv);
   const float ux = dx * dinv, uy = dy * dinv, uz = dz * dinv;
@@ -1022,6 +1039,138 @@ __device__ __forceinline__ float3 angular_edge_force(const ModelParams& p, const
   const float uv = ux * vx + uy * vy + uz * vz;
   return make_float3(SB * ux + (vx - uv * ux) * dinv, SB * uy + (vy - uv * uy) * dinv,
                      SB * uz + (vz - uv * uz) * dinv);
+}
+
+// The same for degrees <= 4, four components at a time: a component's A and B are
+// used as soon as they are summed over n, so no array of them stays live (A and
+// B whole took 48 registers; mixed-mode descriptor stage of 200k carbon 0.724
+// -> 0.659 ms, FP32 about the same).  Two edges per lane at once, which read each
+// moment derivative once for both, were no faster (1M carbon 3.35 against 3.33
+// ms, copper with its 18 edges per atom 2.40 against 2.33).
+template <int KM, int NAM, bool AG, bool FAST, bool EX>
+__device__ __forceinline__ float3 angular_edge_force4(const ModelParams& p, int t1,
+                                                     const float* ctab,
+                                                     const float* __restrict__ av,
+                                                     const float4& e)
+{
+  constexpr int KP = (KM + 3) & ~3;
+  constexpr int NLM = kNumLM;
+  const int nA = EX ? NAM : p.nA;
+  const int nlm = EX ? NLM : (p.L_max + 1) * (p.L_max + 1) - 1;
+  const int t2 = row_type(e);
+  float d, dinv, rc, rcinv, fc, fcp;
+  pair_cutoff<FAST>(p, 1, t1, t2, rc, rcinv);
+  edge_length<FAST>(e.x * e.x + e.y * e.y + e.z * e.z, d, dinv);
+  const float ux = e.x * dinv, uy = e.y * dinv, uz = e.z * dinv;
+  cutoff_fc<FAST>(rc, rcinv, d, fc, fcp);
+  float2 g[NAM], gp[NAM];   // g_n, g'_n in both halves of a pair
+  {
+    float fn[KP], fnp[KP];
+#pragma unroll
+    for (int kk = 0; kk < KP; ++kk) fn[kk] = fnp[kk] = 0.0f;
+    radial_basis_d<KM>(p.kA, rcinv, d, fc, fcp, fn, fnp);
+    const float* c = ctab + t2 * nA * KP;
+#pragma unroll
+    for (int n = 0; n < NAM; ++n) {
+      if (n < nA) {
+        const float gn = dot_basis<KM>(c + n * KP, fn), gpn = dot_basis<KM>(c + n * KP, fnp);
+        g[n] = make_float2(gn, gn);
+        gp[n] = make_float2(gpn, gpn);
+      }
+    }
+  }
+  // powers of u_z and of u_x + i u_y
+  float zp[5], re[5], im[5];
+  zp[0] = re[0] = 1.0f;
+  im[0] = 0.0f;
+#pragma unroll
+  for (int m = 1; m < 5; ++m) {
+    zp[m] = zp[m - 1] * uz;
+    re[m] = ux * re[m - 1] - uy * im[m - 1];
+    im[m] = ux * im[m - 1] + uy * re[m - 1];
+  }
+  float SB = 0.0f, vx = 0.0f, vy = 0.0f, vz = 0.0f;
+  float A[NLM], B[NLM];
+#pragma unroll
+  for (int q = 0; q < NLM / 4; ++q) {
+    if (!EX && 4 * q >= nlm) break;
+    float2 a2[2], b2[2];
+    a2[0] = a2[1] = b2[0] = b2[1] = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int n = 0; n < NAM; ++n) {
+      if (n < nA) {
+        const float4* an = reinterpret_cast<const float4*>(av + n * NLM) + q;
+        const float4 a4 = AG ? __ldg(an) : *an;
+        const float2 lo = make_float2(a4.x, a4.y), hi = make_float2(a4.z, a4.w);
+        a2[0] = fma2(lo, g[n], a2[0]);
+        a2[1] = fma2(hi, g[n], a2[1]);
+        b2[0] = fma2(lo, gp[n], b2[0]);
+        b2[1] = fma2(hi, gp[n], b2[1]);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      A[4 * q + 2 * h] = a2[h].x;
+      A[4 * q + 2 * h + 1] = a2[h].y;
+      B[4 * q + 2 * h] = b2[h].x;
+      B[4 * q + 2 * h + 1] = b2[h].y;
+    }
+    // the components whose (re, im) pair ends in this four
+    int idx = 0;
+#pragma unroll
+    for (int L = 1; L <= 4; ++L) {
+#pragma unroll
+      for (int m = 0; m <= L; ++m) {
+        const int last = m == 0 ? idx : idx + 1;
+        if (last / 4 == q) {
+          float dzf;
+          const float zf = zpoly(L, m, zp, &dzf);
+          if (m == 0) {
+            SB += B[idx] * zf;
+            vz += A[idx] * dzf;
+          } else {
+            const float Ar = A[idx], Ai = A[idx + 1];
+            const float mzf = m * zf;
+            SB += (B[idx] * re[m] + B[idx + 1] * im[m]) * zf;
+            vx += mzf * (Ar * re[m - 1] + Ai * im[m - 1]);
+            vy += mzf * (Ai * re[m - 1] - Ar * im[m - 1]);
+            vz += dzf * (Ar * re[m] + Ai * im[m]);
+          }
+        }
+        idx = last + 1;
+      }
+    }
+  }
+  const float uv = ux * vx + uy * vy + uz * vz;
+  return make_float3(SB * ux + (vx - uv * ux) * dinv, SB * uy + (vy - uv * uy) * dinv,
+                     SB * uz + (vz - uv * uz) * dinv);
+}
+
+// Forces of the edges erow[0 .. na) of one center into frow (which may be the
+// same memory: each lane reads an edge before it writes the force), by the G
+// lanes of a group, the next edge loaded one iteration early.
+template <int G, int KM, int NAM, int LMAX, bool AG, bool FAST, bool EX>
+__device__ __forceinline__ void angular_force_row(const ModelParams& p, int t1, const float* ctab,
+                                                  const float* __restrict__ av, int na, int gl,
+                                                  const float4* erow, float4* frow)
+{
+  float4 next = make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+  if (gl < na) next = erow[gl];
+  for (int k = gl; k < na; k += G) {
+    const float4 e = next;
+    if (k + G < na) next = erow[k + G];
+    float3 f;
+    if constexpr (LMAX <= 4) {
+      f = angular_edge_force4<KM, NAM, AG, FAST, EX>(p, t1, ctab, av, e);
+    } else {
+      const int t2 = row_type(e);
+      float rc, rcinv;
+      pair_cutoff<FAST>(p, 1, t1, t2, rc, rcinv);
+      f = angular_edge_force<KM, NAM, LMAX, AG, FAST>(
+        p, ctab + t2 * p.nA * ((KM + 3) & ~3), av, rc, rcinv, e.x, e.y, e.z);
+    }
+    frow[k] = make_float4(f.x, f.y, f.z, 0.0f);
+  }
 }
 
 // NRM/KM/NAM: compile-time bounds of nR, basis size + 1, nA for this instance.
@@ -1389,18 +1538,7 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
     // place of its edge
     const float* ctab = sm + Lay.c_ang + t1 * T * nA * Lay.kpa;
     float4* frow = f12 + static_cast<size_t>(i) * mn_a;
-    float4 e_next = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (gl < na) e_next = frow[gl];
-    for (int k = gl; k < na; k += G) {
-      const float4 e = e_next;
-      if (k + G < na) e_next = frow[k + G];
-      const int t2 = row_type(e);
-      float rc, rcinv;
-      pair_cutoff<FAST>(p, 1, t1, t2, rc, rcinv);
-      const float3 f = angular_edge_force<KM, NAM, LMAX, false, FAST, EX>(
-        p, ctab + t2 * nA * Lay.kpa, s_a, rc, rcinv, e.x, e.y, e.z);
-      frow[k] = make_float4(f.x, f.y, f.z, 0.0f);
-    }
+    angular_force_row<G, KM, NAM, LMAX, false, FAST, EX>(p, t1, ctab, s_a, na, gl, frow, frow);
   }
 }
 
@@ -1446,15 +1584,8 @@ k_angular_f12(const ModelParams p, int N, const Site* __restrict__ sites,
   float4* frow = f12 + static_cast<size_t>(i) * mn_a;
   // Verlet rows: k_filter_radial left the edge in the slot of its force
   const float4* erow = XR ? ea + static_cast<size_t>(i) * mn_a : frow;
-  for (int k = gl; k < na; k += G) {
-    const float4 e = erow[k];
-    const int t2 = row_type(e);
-    float rc, rcinv;
-    pair_cutoff<FAST>(p, 1, t1, t2, rc, rcinv);
-    const float3 f = angular_edge_force<KM, NAM, LMAX, true, FAST>(
-      p, sm + (t1 * T + t2) * nA * KP, ai, rc, rcinv, e.x, e.y, e.z);
-    frow[k] = make_float4(f.x, f.y, f.z, 0.0f);
-  }
+  angular_force_row<G, KM, NAM, LMAX, true, FAST, false>(p, t1, sm + t1 * T * nA * KP, ai, na, gl,
+                                                         erow, frow);
 }
 
 // ---------------------------------------------------------------------------
@@ -1599,16 +1730,26 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
             atomicOr(&st->overflow, 4);
           }
         } else {
-          float rc, rcinv;
-          pair_cutoff<FAST>(p, 1, t1, t2, rc, rcinv);
           const int nA = p.nA;
           constexpr int NLM = num_lm<LMAX>();
-          const float3 fij = angular_edge_force<KM, NAM, LMAX, true, FAST>(
-            p, sm + (t1 * T + t2) * nA * KP, acoef + static_cast<size_t>(i) * nA * NLM, rc,
-            rcinv, dx, dy, dz);
-          const float3 fji = angular_edge_force<KM, NAM, LMAX, true, FAST>(
-            p, sm + (t2 * T + t1) * nA * KP, acoef + static_cast<size_t>(j) * nA * NLM, rc,
-            rcinv, -dx, -dy, -dz);
+          const float* av_i = acoef + static_cast<size_t>(i) * nA * NLM;
+          const float* av_j = acoef + static_cast<size_t>(j) * nA * NLM;
+          float3 fij, fji;
+          if constexpr (LMAX <= 4) {
+            const float4 back =
+              make_float4(-dx, -dy, -dz, __int_as_float(t1 << kRowTypeShift));
+            fij = angular_edge_force4<KM, NAM, true, FAST, false>(p, t1, sm + t1 * T * nA * KP,
+                                                                 av_i, e);
+            fji = angular_edge_force4<KM, NAM, true, FAST, false>(p, t2, sm + t2 * T * nA * KP,
+                                                                 av_j, back);
+          } else {
+            float rc, rcinv;
+            pair_cutoff<FAST>(p, 1, t1, t2, rc, rcinv);
+            fij = angular_edge_force<KM, NAM, LMAX, true, FAST>(
+              p, sm + (t1 * T + t2) * nA * KP, av_i, rc, rcinv, dx, dy, dz);
+            fji = angular_edge_force<KM, NAM, LMAX, true, FAST>(
+              p, sm + (t2 * T + t1) * nA * KP, av_j, rc, rcinv, -dx, -dy, -dz);
+          }
           a12 = make_float4(fij.x, fij.y, fij.z, 0.0f);
           a21 = make_float4(fji.x, fji.y, fji.z, 0.0f);
         }
@@ -1765,18 +1906,19 @@ void launch_filter_tf(Engine& e, int N, cudaStream_t s)
   constexpr int APB = kBlock / G, KP = (KM + 3) & ~3;
   const ModelParams& p = e.params;
   const int blocks = (N + APB - 1) / APB;
-  if (filter_bins(p, KP)) {
+  auto launch = [&](auto kernel, size_t bin_float4) {
     const size_t smem =
-      sizeof(float) * (filter_table_floats(p, KP) + 4 * kBlock * filter_bin_float4(p, KP));
-    k_filter_radial<G, NRM, KM, true, FAST><<<blocks, kBlock, smem, s>>>(
-      p, N, e.d_box, e.scratch.sites, e.d_nstate, nb.nn_v, nb.nl_v, nb.mn_v, nb.nn_r, nb.nl_r,
-      nb.mn_r, nb.nn_a, nb.nl_a, nb.mn_a, e.scratch.f12, e.scratch.qrad);
-  } else {
-    const size_t smem = sizeof(float) * filter_table_floats(p, KP);
-    k_filter_radial<G, NRM, KM, false, FAST><<<blocks, kBlock, smem, s>>>(
-      p, N, e.d_box, e.scratch.sites, e.d_nstate, nb.nn_v, nb.nl_v, nb.mn_v, nb.nn_r, nb.nl_r,
-      nb.mn_r, nb.nn_a, nb.nl_a, nb.mn_a, e.scratch.f12, e.scratch.qrad);
-  }
+      sizeof(float) * (filter_table_floats(p, KP) + 4 * kBlock * bin_float4);
+    kernel<<<blocks, kBlock, smem, s>>>(p, N, e.d_box, e.scratch.sites, e.d_nstate, nb.nn_v,
+                                        nb.nl_v, nb.mn_v, nb.nn_r, nb.nl_r, nb.mn_r, nb.nn_a,
+                                        nb.nl_a, nb.mn_a, e.scratch.f12, e.scratch.qrad);
+  };
+  const int bin = filter_bin<KM>(p);
+  if (bin == kBinShared)
+    launch(k_filter_radial<G, NRM, KM, kBinShared, FAST>, filter_bin_float4(p, KP));
+  else if (bin == kBinNone) launch(k_filter_radial<G, NRM, KM, kBinNone, FAST>, 0);
+  if constexpr (KM <= 9)
+    if (bin == kBinRegs) launch(k_filter_radial<G, NRM, KM, kBinRegs, FAST>, 0);
 }
 
 template <int G, int NRM, int KM>
