@@ -1253,7 +1253,6 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
   float* s_a = mine + Lay.a;
   float* s_q = mine + Lay.q;
   float* s_fp = mine + Lay.fp;
-  float* s_gh = mine + Lay.gh;
   const int t1 = active ? static_cast<int>(sites[i].type) : 0;
 
   // ---- 1. filter the Verlet row, radial descriptors -------------------------
@@ -1436,86 +1435,94 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
     __syncwarp();
     tc_ann<APB, G>(p, Lay, sm, slot, gl, active, t1, i, s_q, pe_ann, st);
   } else {
-    for (int h = H + gl; h < p.H4; h += G) s_gh[h] = 0.0f;
+    // In this stage adjacent lanes take different centers of the warp and the
+    // same hidden units (ag: this lane's share of them): a 16-byte read of the
+    // weights is then the same for the lanes of one type, which costs the
+    // shared-memory pipe 2.3 cycles, where four lanes of a center with four
+    // rows each took 4 (forward) and, at the rows' common bank, 8 (backward).
+    const int ac = lane % APW, ag = lane / APW;
+    const int a_slot = warp * APW + ac, a_i = blockIdx.x * APB + a_slot;
+    const bool a_active = a_i < N;
+    const int a_t = __shfl_sync(kFull, t1, ac * G);
+    float* a_mine = sm + Lay.atoms_base + a_slot * Lay.per_atom;
+    const float* a_q = a_mine + Lay.q;
+    float* a_fp = a_mine + Lay.fp;
+    float* a_gh = a_mine + Lay.gh;
+    for (int h = H + ag; h < p.H4; h += G) a_gh[h] = 0.0f;
     __syncwarp();
     const float* w0t = Lay.wt >= 0 ? sm + Lay.wt : p.w0t;
+    const int hq = p.H4 / 4;
+    const float4* wt = reinterpret_cast<const float4*>(w0t + static_cast<size_t>(a_t) * dim * p.H4);
     float e_part = 0.0f;
-    if (active) {
+    if (a_active) {
       // hidden layer: each lane owns two groups of four consecutive hidden units
-      // (float4 rows of the transposed w0; eight independent FMA chains in one
+      // (float4 rows of the transposed w0; four chains of packed pairs in one
       // pass, each sequential in d as in the reference)
-      const int hq = p.H4 / 4;
-      const float4* wt =
-        reinterpret_cast<const float4*>(w0t + static_cast<size_t>(t1) * dim * p.H4);
       auto finish = [&](int h, float z) {
         if (h < H) {
-          const float x1 = tanhf(z - __ldg(p.b0 + t1 * H + h));
-          const float w1 = __ldg(p.w1 + t1 * H + h);
+          const float x1 = tanhf(z - __ldg(p.b0 + a_t * H + h));
+          const float w1 = __ldg(p.w1 + a_t * H + h);
           e_part += w1 * x1;
-          s_gh[h] = w1 * (1.0f - x1 * x1);
+          a_gh[h] = w1 * (1.0f - x1 * x1);
         }
       };
-      for (int h4 = gl; h4 < hq; h4 += 2 * G) {
+      for (int h4 = ag; h4 < hq; h4 += 2 * G) {
         const bool has_b = h4 + G < hq;
         const int h4b = has_b ? h4 + G : h4;   // past the end: computed, dropped
-        float z0 = 0.0f, z1 = 0.0f, z2 = 0.0f, z3 = 0.0f;
-        float z4 = 0.0f, z5 = 0.0f, z6 = 0.0f, z7 = 0.0f;
-#pragma unroll 2
+        float2 z01 = make_float2(0.0f, 0.0f), z23 = z01, z45 = z01, z67 = z01;
+#pragma unroll 4
         for (int d = 0; d < dim; ++d) {
-          const float q = s_q[d];
+          const float q = a_q[d];
+          const float2 q2 = make_float2(q, q);
           const float4 wa = wt[d * hq + h4];
           const float4 wb = wt[d * hq + h4b];
-          z0 = fmaf(wa.x, q, z0);
-          z1 = fmaf(wa.y, q, z1);
-          z2 = fmaf(wa.z, q, z2);
-          z3 = fmaf(wa.w, q, z3);
-          z4 = fmaf(wb.x, q, z4);
-          z5 = fmaf(wb.y, q, z5);
-          z6 = fmaf(wb.z, q, z6);
-          z7 = fmaf(wb.w, q, z7);
+          z01 = fma2(make_float2(wa.x, wa.y), q2, z01);
+          z23 = fma2(make_float2(wa.z, wa.w), q2, z23);
+          z45 = fma2(make_float2(wb.x, wb.y), q2, z45);
+          z67 = fma2(make_float2(wb.z, wb.w), q2, z67);
         }
-        finish(4 * h4, z0);
-        finish(4 * h4 + 1, z1);
-        finish(4 * h4 + 2, z2);
-        finish(4 * h4 + 3, z3);
+        finish(4 * h4, z01.x);
+        finish(4 * h4 + 1, z01.y);
+        finish(4 * h4 + 2, z23.x);
+        finish(4 * h4 + 3, z23.y);
         if (has_b) {
-          finish(4 * h4b, z4);
-          finish(4 * h4b + 1, z5);
-          finish(4 * h4b + 2, z6);
-          finish(4 * h4b + 3, z7);
+          finish(4 * h4b, z45.x);
+          finish(4 * h4b + 1, z45.y);
+          finish(4 * h4b + 2, z67.x);
+          finish(4 * h4b + 3, z67.y);
         }
       }
     }
-    e_part = group_sum<G>(e_part);
-    if (active && gl == 0) pe_ann[i] = static_cast<double>(e_part - __ldg(p.out_bias + t1));
+#pragma unroll
+    for (int o = APW; o < 32; o <<= 1) e_part += __shfl_xor_sync(kFull, e_part, o);
+    if (a_active && ag == 0) pe_ann[a_i] = static_cast<double>(e_part - __ldg(p.out_bias + a_t));
     __syncwarp();
-    if (active) {
+    if (a_active) {
       // dE/dq: four descriptor components per lane at once (d0, d0 + G,
-      // d0 + 2G, d0 + 3G), float4 over h, each sum in the same order as before
-      const int hq = p.H4 / 4;
-      const float4* g4 = reinterpret_cast<const float4*>(s_gh);
-      const float4* wt =
-        reinterpret_cast<const float4*>(w0t + static_cast<size_t>(t1) * dim * p.H4);
-      for (int d0 = gl; d0 < dim; d0 += 4 * G) {
+      // d0 + 2G, d0 + 3G), float4 over h, even and odd hidden units apart
+      const float4* g4 = reinterpret_cast<const float4*>(a_gh);
+      for (int d0 = ag; d0 < dim; d0 += 4 * G) {
         int dd[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) dd[k] = min(d0 + k * G, dim - 1);   // past dim: dropped
-        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float2 acc[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[k] = make_float2(0.0f, 0.0f);
 #pragma unroll 2
         for (int h = 0; h < hq; ++h) {
           const float4 g = g4[h];
+          const float2 g01 = make_float2(g.x, g.y), g23 = make_float2(g.z, g.w);
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const float4 w = wt[dd[k] * hq + h];
-            acc[k] = fmaf(g.x, w.x, acc[k]);
-            acc[k] = fmaf(g.y, w.y, acc[k]);
-            acc[k] = fmaf(g.z, w.z, acc[k]);
-            acc[k] = fmaf(g.w, w.w, acc[k]);
+            acc[k] = fma2(g01, make_float2(w.x, w.y), acc[k]);
+            acc[k] = fma2(g23, make_float2(w.z, w.w), acc[k]);
           }
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          if (d0 + k * G < dim) s_fp[d0 + k * G] = acc[k] * __ldg(p.q_scaler + d0 + k * G);
+          if (d0 + k * G < dim)
+            a_fp[d0 + k * G] = (acc[k].x + acc[k].y) * __ldg(p.q_scaler + d0 + k * G);
       }
     }
     __syncwarp();
