@@ -303,9 +303,9 @@ int nepx_get_tuning(nepx_t* h, int* v, int* tuned)
 int nepx_set_tuning(nepx_t* h, const int* v)
 {
   if (!h || !v) return NEPX_ERR_ARG;
-  auto lanes = [](int g) { return g == 4 || g == 8; };
-  if (!lanes(v[0]) || !lanes(v[1]) || !(v[2] == 3 || v[2] == 4) || !lanes(v[3]) ||
-      !lanes(v[4]) || !(v[5] == 0 || v[5] == 1) || !(v[6] == 3 || v[6] == 4))
+  using nepx::lanes_built;
+  if (!lanes_built(v[0]) || !lanes_built(v[1]) || !(v[2] == 3 || v[2] == 4) ||
+      !lanes_built(v[3]) || !lanes_built(v[4]) || !(v[5] == 0 || v[5] == 1) || !(v[6] == 3 || v[6] == 4))
     return fail(h, NEPX_ERR_ARG, "launch choice outside the built variants");
   nepx::Engine& e = h->engine;
   e.filter_group = v[0];

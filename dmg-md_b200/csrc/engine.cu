@@ -265,9 +265,8 @@ void tune_load_file()
     ok = ok && static_cast<bool>(ls >> v.filter_group >> v.group >> v.fused_minb >> v.f12_group >>
                                  v.gather_group >> v.fuse_f12 >> v.gather_minb);
     // only the shapes the launchers instantiate; anything else is ignored
-    auto lanes = [](int g) { return g == 4 || g == 8; };
-    ok = ok && lanes(v.filter_group) && lanes(v.group) && lanes(v.f12_group) &&
-         lanes(v.gather_group) && (v.fused_minb == 3 || v.fused_minb == 4) &&
+    ok = ok && lanes_built(v.filter_group) && lanes_built(v.group) && lanes_built(v.f12_group) &&
+         lanes_built(v.gather_group) && (v.fused_minb == 3 || v.fused_minb == 4) &&
          (v.fuse_f12 == 0 || v.fuse_f12 == 1) && (v.gather_minb == 3 || v.gather_minb == 4);
     if (ok) g_tune.emplace_back(k, v);
   }
@@ -316,124 +315,121 @@ void engine_autotune(Engine& e, int N, const double* pos, const int* type, cudaS
     e.tuned = true;
     return;
   }
-  // candidate lanes per center; each variant runs 3 times, the median counts
-  const int groups[2] = {4, 8};
-  float best_f = 1e30f, best_g = 1e30f;
-  int pick_f = e.group, pick_g = e.gather_group;
-  cudaEvent_t a, b, c;
+  if (N < kWideAtoms) {
+    // a small system: lanes by size, nothing timed.  A kernel's time is then the
+    // chain of one center's edges plus what each center costs the chip, and the
+    // best group narrows as the atoms fill it (us, lanes 4 8 16 32, the other
+    // kernel at 8):
+    //   descriptor kernel   water 210: 32 21 17 14;  carbon 1,000: 32 28 26 28;
+    //                       4,096: 36 34 40 51;  8,000: 44 48 56 77
+    //   filter              water 600: 45 34 28 26;  1,551: 50 38 32 32;
+    //                       carbon 4,096: 36 34 34 38;  8,000: 50 48 54 63
+    //   gather              water 1,551: 44 30 23 14;  carbon 4,096: 34 24 21 19;
+    //                       8,000: 35 25 29 26
+    // (1,551 water atoms in the descriptor kernel: 44 38 38 36.)  A rule also
+    // gives every process of a small system the same sums; its lines are powers of
+    // two because the picks are kept by size class.
+    e.filter_group = N < 1024 ? 32 : 16;
+    e.group = !fused_wide_groups(e) ? 8 : N < 512 ? 32 : N < 1024 ? 16 : 8;
+    e.fused_minb = 3;
+    e.f12_group = 8;
+    e.gather_group = 32;
+    e.gather_minb = 3;
+    e.fuse_f12 = true;
+    e.fuse_f12 = fused_angular_force(e);
+    e.tuned = true;
+    tune_store(key, TuneVal{e.filter_group, e.group, e.fused_minb, e.f12_group, e.gather_group,
+                            e.fuse_f12 ? 1 : 0, e.gather_minb});
+    return;
+  }
+  const int groups[2] = {4, 8};   // candidate lanes per center
+  cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);
-  cudaEventCreate(&c);
-  int pick_a = e.f12_group;
+  // each variant: one untimed launch (it pays for its instruction cache and
+  // the rows' way into L2), then the median of `reps`
+  auto median = [&](int reps, auto&& launch) {
+    float t[5];
+    launch();
+    for (int r = 0; r < reps; ++r) {
+      cudaEventRecord(a, stream);
+      launch();
+      cudaEventRecord(b, stream);
+      cudaEventSynchronize(b);
+      cudaEventElapsedTime(&t[r], a, b);
+    }
+    std::sort(t, t + reps);
+    return t[reps / 2];
+  };
   if (!e.use_xr) {
     float best = 1e30f;
     int pick = e.filter_group;
-    // each grouping: one untimed launch, then the median of five
     for (int g : groups) {
       e.filter_group = g;
-      float t[6];
-      for (int r = 0; r < 6; ++r) {
-        cudaEventRecord(a, stream);
-        launch_filter(e, N, stream);
-        cudaEventRecord(b, stream);
-        cudaEventSynchronize(b);
-        cudaEventElapsedTime(&t[r], a, b);
-      }
-      std::sort(t + 1, t + 6);
-      if (t[3] < best) {
-        best = t[3];
-        pick = g;
+      const float t = median(5, [&] { launch_filter(e, N, stream); });
+      if (t < best) {
+        best = t;
+        pick = e.filter_group;
       }
     }
     e.filter_group = pick;
   }
-  // the descriptor kernel's occupancy builds (CTAs per SM), when the shape has
-  // two (the FP32 build of the small shape; the tensor-core build comes at 3)
-  const int minbs[2] = {3, 4};
+  // the descriptor kernel's lanes per center, its occupancy builds (CTAs per
+  // SM) where the shape has two (the FP32 build of the small shape; the
+  // tensor-core build comes at 3), and the angular partial
+  // forces inside it (small shape, Verlet rows) or in their own kernel, whose
+  // lanes per center vary too
   const int n_minb = (fused_occupancy_variants(e.params) && e.precision == 0) ? 2 : 1;
-  if (n_minb == 1) e.fused_minb = 3;
-  int pick_m = e.fused_minb;
-  // the descriptor kernel with and without the angular partial forces (the
-  // fused form exists for the small shape on Verlet rows)
   e.fuse_f12 = true;
   const int n_ff = fused_angular_force(e) ? 2 : 1;
-  e.fuse_f12 = false;
+  float best_f = 1e30f;
+  int pick_f = 8, pick_m = 3, pick_a = 4;
   bool pick_ff = false;
   for (int ff = 0; ff < n_ff; ++ff)
-  for (int gf : groups) {
-    for (int mi = 0; mi < n_minb; ++mi)
-    for (int gg : groups) {
-      e.fuse_f12 = ff == 1;
-      e.group = gf;
-      e.fused_minb = minbs[mi];
-      e.f12_group = gg;   // angular-force grouping varies together with the gather's
-      e.gather_group = gg;
-      // with the fused form the angular-force grouping plays no part (the
-      // gather's groupings are timed with the separate form)
-      if (e.fuse_f12 && gg != groups[0]) continue;
-      float tf[3], tg[3];
-      // one untimed call first: each build's first launch pays for its
-      // instruction cache and the rows' way into L2
-      launch_descriptor(e, N, pos, type, stream);
-      for (int r = 0; r < 3; ++r) {
-        cudaEventRecord(a, stream);
-        launch_descriptor(e, N, pos, type, stream);
-        cudaEventRecord(b, stream);
-        double* out = e.scratch.tune_out;   // 13 N doubles: pe, force, virial
+    for (int g : groups)
+      for (int mi = 0; mi < n_minb; ++mi)
+        for (int gg = 4; gg <= 8; gg += 4) {
+          e.fuse_f12 = ff == 1;
+          e.group = g;
+          e.fused_minb = mi == 0 ? 3 : 4;
+          e.f12_group = gg;
+          // no angular-force kernel runs: the fused form, and a single system
+          // on explicit rows
+          if (gg > 4 && (e.fuse_f12 || (e.use_xr && e.xr.from_box))) continue;
+          const float t = median(3, [&] { launch_descriptor(e, N, pos, type, stream); });
+          if (t < best_f) {
+            best_f = t;
+            pick_f = e.group;
+            pick_m = e.fused_minb;
+            pick_a = gg;
+            pick_ff = e.fuse_f12;
+          }
+        }
+  // the gather's lanes per center and, on Verlet rows, its two occupancy
+  // builds (the rows, alpha and f12 of the last descriptor call serve every
+  // variant; short kernels: the picks must not follow single launches' noise)
+  float best_g = 1e30f;
+  int pick_g = 8, pick_gm = 3;
+  const int gm_last = !e.use_xr && e.params.L_max <= 4 ? 4 : 3;
+  const int gather_lanes[3] = {4, 8, 32};   // 8,000 carbon atoms: 35 25 23 us
+  const int n_lanes = N < 16384 ? 3 : 2;
+  for (int gm = 3; gm <= gm_last; ++gm)
+    for (int k = 0; k < n_lanes; ++k) {
+      e.gather_minb = gm;
+      e.gather_group = gather_lanes[k];
+      double* out = e.scratch.tune_out;   // 13 N doubles: pe, force, virial
+      const float t = median(5, [&] {
         launch_gather(e, N, pos, type, out, out + N, out + 4 * static_cast<size_t>(N), false,
                       stream);
-        cudaEventRecord(c, stream);
-        cudaEventSynchronize(c);
-        cudaEventElapsedTime(&tf[r], a, b);
-        cudaEventElapsedTime(&tg[r], b, c);
-      }
-      std::sort(tf, tf + 3);
-      std::sort(tg, tg + 3);
-      if (tf[1] < best_f) {
-        best_f = tf[1];
-        pick_f = gf;
-        pick_m = e.fused_minb;
-        pick_a = gg;
-        pick_ff = e.fuse_f12;
-      }
-      if (tg[1] < best_g) {
-        best_g = tg[1];
-        pick_g = gg;
+      });
+      if (t < best_g) {
+        best_g = t;
+        pick_g = e.gather_group;
+        pick_gm = gm;
       }
     }
-  }
-  // the Verlet-row gather's two occupancy builds, with each grouping (the
-  // rows, alpha and f12 of the last descriptor call serve every variant)
-  int pick_gm = 3;
-  if (!e.use_xr && e.params.L_max <= 4) {
-    best_g = 1e30f;
-    for (int gm = 3; gm <= 4; ++gm)
-      for (int gg : groups) {
-        e.gather_minb = gm;
-        e.gather_group = gg;
-        // one untimed launch, then the median of five (short kernels: the
-        // picks must not follow the noise of single launches)
-        float tg[6];
-        for (int r = 0; r < 6; ++r) {
-          cudaEventRecord(a, stream);
-          double* out = e.scratch.tune_out;
-          launch_gather(e, N, pos, type, out, out + N, out + 4 * static_cast<size_t>(N), false,
-                        stream);
-          cudaEventRecord(b, stream);
-          cudaEventSynchronize(b);
-          cudaEventElapsedTime(&tg[r], a, b);
-        }
-        std::sort(tg + 1, tg + 6);
-        if (tg[3] < best_g) {
-          best_g = tg[3];
-          pick_g = gg;
-          pick_gm = gm;
-        }
-      }
-  }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
-  cudaEventDestroy(c);
   e.gather_minb = pick_gm;
   e.group = pick_f;
   e.fused_minb = pick_m;

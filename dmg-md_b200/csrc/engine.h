@@ -131,6 +131,15 @@ int basis_stride(const ModelParams& p);
 size_t fused_smem_bytes(const ModelParams& p);
 // The same for the tensor-core (mixed-precision) build; needs the tc_* fields.
 size_t fused_tc_smem_bytes(const ModelParams& p);
+// Lane groups per center that kernels are built for; 16 and 32 run as 8 where
+// a kernel has no build for the model.
+inline bool lanes_built(int g) { return g == 4 || g == 8 || g == 16 || g == 32; }
+// Systems below this many atoms take their lanes from a rule on the size
+// (engine_autotune); from there on the chip is full at 4 or 8 lanes.
+constexpr int kWideAtoms = 4096;
+// True when the descriptor kernel has 16- and 32-lane groups for this model
+// and precision.
+bool fused_wide_groups(const Engine& e);
 // True when the descriptor kernel comes in two occupancy builds (3 or 4 CTAs
 // per SM, Engine::fused_minb) for this model's shape.
 bool fused_occupancy_variants(const ModelParams& p);
@@ -139,7 +148,8 @@ bool fused_occupancy_variants(const ModelParams& p);
 bool fused_angular_force(const Engine& e);
 void set_fused_smem_limits(const ModelParams& p);
 
-// Times each kernel variant on the given system (a few calls each, stream
+// Takes the lanes of a small system (below kWideAtoms) from its size; otherwise
+// times each kernel variant on the given system (a few calls each, stream
 // synchronised) and keeps the fastest: the lane-group size of the filter,
 // descriptor, angular-force and gather kernels, the CTAs per SM of the
 // descriptor kernel and of the gather, and whether the descriptor kernel

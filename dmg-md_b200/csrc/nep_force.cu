@@ -418,7 +418,8 @@ template <int G>
 __device__ __forceinline__ unsigned group_ballot(bool pred, int group)
 {
   const unsigned b = __ballot_sync(kFull, pred);
-  return (b >> (group * G)) & ((1u << G) - 1u);
+  if constexpr (G == 32) return b;
+  else return (b >> (group * G)) & ((1u << G) - 1u);
 }
 
 template <int G>
@@ -448,18 +449,27 @@ __device__ __forceinline__ void rs_step(float* v, int gl, int& base)
 template <int G, int L>
 __device__ __forceinline__ int reduce_scatter(float* v, int gl)
 {
-  static_assert(G == 2 || G == 4 || G == 8, "group of 2, 4 or 8 lanes");
+  static_assert(G == 4 || G == 8 || G == 16 || G == 32, "group of 4 to 32 lanes");
   static_assert(L % G == 0, "share must divide evenly");
   int base = 0;
-  if constexpr (G == 8) {
+  if constexpr (G == 32) {
+    rs_step<L, 16>(v, gl, base);
+    rs_step<L / 2, 8>(v, gl, base);
+    rs_step<L / 4, 4>(v, gl, base);
+    rs_step<L / 8, 2>(v, gl, base);
+    rs_step<L / 16, 1>(v, gl, base);
+  } else if constexpr (G == 16) {
+    rs_step<L, 8>(v, gl, base);
+    rs_step<L / 2, 4>(v, gl, base);
+    rs_step<L / 4, 2>(v, gl, base);
+    rs_step<L / 8, 1>(v, gl, base);
+  } else if constexpr (G == 8) {
     rs_step<L, 4>(v, gl, base);
     rs_step<L / 2, 2>(v, gl, base);
     rs_step<L / 4, 1>(v, gl, base);
-  } else if constexpr (G == 4) {
+  } else {
     rs_step<L, 2>(v, gl, base);
     rs_step<L / 2, 1>(v, gl, base);
-  } else {
-    rs_step<L, 1>(v, gl, base);
   }
   return base;
 }
@@ -1317,9 +1327,11 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
   // loaded one iteration early
   const float4* earow = (XR ? ea : f12) + static_cast<size_t>(i) * mn_a;
   for (int nc = 0; nc < nA; nc += CN) {
-    float v[CN * NLM];
+    // padded to a whole share per lane
+    constexpr int VL = (CN * NLM + G - 1) / G * G;
+    float v[VL];
 #pragma unroll
-    for (int q = 0; q < CN * NLM; ++q) v[q] = 0.0f;
+    for (int q = 0; q < VL; ++q) v[q] = 0.0f;
     float4 e_next = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (gl < na) e_next = earow[gl];
     for (int base = 0; base < na_max; base += G) {
@@ -1370,8 +1382,8 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
         }
       }
     }
-    const int at = reduce_scatter<G, CN * NLM>(v, gl);
-    constexpr int share = CN * NLM / G;
+    const int at = reduce_scatter<G, VL>(v, gl);
+    constexpr int share = VL / G;
     const int lim = (nA - nc < CN ? nA - nc : CN) * NLM;
 #pragma unroll
     for (int q = 0; q < share; ++q)
@@ -1889,6 +1901,11 @@ void launch_fused_tx(Engine& e, int N, cudaStream_t s)
     e.xr.ea, e.scratch.qrad, e.scratch.alpha, e.scratch.acoef, e.scratch.f12, e.scratch.pe_ann);
 }
 
+// Groups of 16 and 32 lanes serve small systems, where a kernel's time is one
+// center's chain of edges and not the chip's throughput (4,096 atoms at 8 lanes
+// are 256 CTAs of 128): FP32 builds of the exact small shape, and the filter and
+// gather of the small shape, chosen by size below kWideAtoms.  Elsewhere they run
+// as groups of 8.
 template <int G, int NRM, int KM, int NAM, bool XR, int LMAX, int MINB, bool TC, bool FF = false>
 void launch_fused_t(Engine& e, int N, cudaStream_t s)
 {
@@ -1990,6 +2007,20 @@ void set_fused_smem_t(const ModelParams& p)
   }
 }
 
+template <int G>
+void set_fused_smem_wide(const ModelParams& p)
+{
+  constexpr int n = kSmallN, k = kSmallK;
+  const int bytes =
+    fused_layout(p, kBlock / G, (k + 3) & ~3, fused_smem_budget(3), false).total_bytes;
+  auto limit = [&](auto kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  };
+  limit(k_nep_fused<G, n, k, n, true, 4, 3, false, false, true>);
+  limit(k_nep_fused<G, n, k, n, false, 4, 3, false, true, true>);
+  limit(k_nep_fused<G, n, k, n, false, 4, 3, false, false, true>);
+}
+
 template <int G, int KM, int NAM, bool XR, int LMAX, int GMINB, bool FAST>
 void launch_gather_tf(Engine& e, int N, double* pe, double* force, double* virial,
                       bool accumulate, cudaStream_t s)
@@ -2059,6 +2090,16 @@ void launch_fused_small(Engine& e, int N, cudaStream_t s)
   }
 }
 
+// groups of 16 and 32: three CTAs per SM, the angular force inside on Verlet rows
+template <int G>
+void launch_fused_wide(Engine& e, int N, cudaStream_t s)
+{
+  constexpr int n = kSmallN, k = kSmallK;
+  if (e.use_xr) launch_fused_tx<G, n, k, n, true, 4, 3, false, false, true>(e, N, s);
+  else if (e.fuse_f12) launch_fused_tx<G, n, k, n, false, 4, 3, false, true, true>(e, N, s);
+  else launch_fused_tx<G, n, k, n, false, 4, 3, false, false, true>(e, N, s);
+}
+
 template <int G, int KM, int NAM, int LMAX>
 void launch_gather_g(Engine& e, int N, double* pe, double* force, double* virial,
                      bool accumulate, cudaStream_t s)
@@ -2077,6 +2118,8 @@ void launch_gather_g(Engine& e, int N, double* pe, double* force, double* virial
 int basis_stride(const ModelParams& p) { return small_shape(p) ? round4(kSmallK) : round4(kMaxBasis); }
 
 bool fused_occupancy_variants(const ModelParams& p) { return small_shape(p); }
+
+bool fused_wide_groups(const Engine& e) { return exact_shape(e.params) && e.precision == 0; }
 
 // Largest dynamic shared memory a descriptor-kernel variant this model runs needs.
 size_t fused_smem_bytes(const ModelParams& p)
@@ -2100,6 +2143,8 @@ void set_fused_smem_limits(const ModelParams& p)
     return;
   }
   if (small_shape(p)) {
+    set_fused_smem_wide<16>(p);
+    set_fused_smem_wide<32>(p);
     set_fused_smem_t<4, kSmallN, kSmallK, kSmallN, 4, 3, false, true>(p);
     set_fused_smem_t<8, kSmallN, kSmallK, kSmallN, 4, 3, false, true>(p);
     set_fused_smem_t<4, kSmallN, kSmallK, kSmallN, 4, 4, false, true>(p);
@@ -2131,7 +2176,9 @@ size_t fused_tc_smem_bytes(const ModelParams& p)
 void launch_filter(Engine& e, int N, cudaStream_t s)
 {
   const bool small = small_shape(e.params);
-  if (e.filter_group == 8) {
+  if (small && e.filter_group == 32) launch_filter_t<32, kSmallN, kSmallK>(e, N, s);
+  else if (small && e.filter_group == 16) launch_filter_t<16, kSmallN, kSmallK>(e, N, s);
+  else if (e.filter_group >= 8) {
     if (small) launch_filter_t<8, kSmallN, kSmallK>(e, N, s);
     else launch_filter_t<8, kMaxN, kMaxBasis>(e, N, s);
   } else {
@@ -2153,7 +2200,9 @@ void launch_descriptor(Engine& e, int N, const double*, const int*, cudaStream_t
   const bool high = high_degree(e.params);
   if (!e.use_xr) launch_filter(e, N, stream);
   if (high) launch_fused_g<kHighFusedGroup, kMaxN, kMaxBasis, kMaxN, 8, 2>(e, N, stream);
-  else if (e.group == 8) {
+  else if (e.group == 32 && fused_wide_groups(e)) launch_fused_wide<32>(e, N, stream);
+  else if (e.group == 16 && fused_wide_groups(e)) launch_fused_wide<16>(e, N, stream);
+  else if (e.group >= 8) {
     if (small) launch_fused_small<8>(e, N, stream);
     else launch_fused_g<8, kMaxN, kMaxBasis, kMaxN, 4, 2>(e, N, stream);
   } else {
@@ -2165,7 +2214,7 @@ void launch_descriptor(Engine& e, int N, const double*, const int*, cudaStream_t
   if (e.use_xr && e.xr.from_box) return;
   if (fused_angular_force(e)) return;   // the descriptor kernel wrote f12
   if (high) launch_f12_t<kHighGroup, kMaxBasis, kMaxN, 8>(e, N, stream);
-  else if (e.f12_group == 8) {
+  else if (e.f12_group >= 8) {
     if (small) launch_f12_t<8, kSmallK, kSmallN, 4>(e, N, stream);
     else launch_f12_t<8, kMaxBasis, kMaxN, 4>(e, N, stream);
   } else {
@@ -2180,6 +2229,10 @@ void launch_gather(Engine& e, int N, const double*, const int*, double* pe, doub
   const bool small = small_shape(e.params);
   if (high_degree(e.params))
     launch_gather_g<kHighGroup, kMaxBasis, kMaxN, 8>(e, N, pe, force, virial, accumulate, stream);
+  else if (small && e.gather_group == 32)
+    launch_gather_g<32, kSmallK, kSmallN, 4>(e, N, pe, force, virial, accumulate, stream);
+  else if (small && e.gather_group == 16)
+    launch_gather_g<16, kSmallK, kSmallN, 4>(e, N, pe, force, virial, accumulate, stream);
   else if (e.gather_group == 4) {
     if (small) launch_gather_g<4, kSmallK, kSmallN, 4>(e, N, pe, force, virial, accumulate, stream);
     else launch_gather_g<4, kMaxBasis, kMaxN, 4>(e, N, pe, force, virial, accumulate, stream);
