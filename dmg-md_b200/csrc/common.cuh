@@ -99,6 +99,55 @@ __device__ __forceinline__ void mic_f32(const Box& b, float& x, float& y, float&
   }
 }
 
+// The same minimum image with the box's numbers laid out for a sweep over
+// neighbours: an orthogonal box's edges and half edges in registers, half an
+// edge being infinite where the direction is not periodic (one comparison and
+// one signed addition per direction, no test of the boundary); a general box's
+// matrix and inverse in shared memory (18 floats), where they cost no registers.
+// The results are mic_f32's bit for bit.
+struct MinImage {
+  float lx, ly, lz, hx, hy, hz;
+  const float* fh;
+  int pbc;
+  bool ortho;
+
+  // Called by every thread of the block, with a barrier before the first use;
+  // s_fh: 18 floats of shared memory.
+  __device__ __forceinline__ MinImage(const Box* __restrict__ b, float* s_fh)
+  {
+    for (int k = threadIdx.x; k < 18; k += blockDim.x) s_fh[k] = b->fh[k];
+    fh = s_fh;
+    lx = b->fh[0];
+    ly = b->fh[4];
+    lz = b->fh[8];
+    const float never = __int_as_float(0x7f800000);
+    hx = b->pbc[0] == 1 ? lx * 0.5f : never;
+    hy = b->pbc[1] == 1 ? ly * 0.5f : never;
+    hz = b->pbc[2] == 1 ? lz * 0.5f : never;
+    pbc = (b->pbc[0] == 1 ? 1 : 0) | (b->pbc[1] == 1 ? 2 : 0) | (b->pbc[2] == 1 ? 4 : 0);
+    ortho = b->ortho != 0;
+  }
+
+  __device__ __forceinline__ void operator()(float& x, float& y, float& z) const
+  {
+    if (ortho) {
+      if (fabsf(x) > hx) x -= copysignf(lx, x);
+      if (fabsf(y) > hy) y -= copysignf(ly, y);
+      if (fabsf(z) > hz) z -= copysignf(lz, z);
+    } else {
+      float sx = fh[9] * x + fh[10] * y + fh[11] * z;
+      float sy = fh[12] * x + fh[13] * y + fh[14] * z;
+      float sz = fh[15] * x + fh[16] * y + fh[17] * z;
+      if (pbc & 1) sx -= nearbyintf(sx);
+      if (pbc & 2) sy -= nearbyintf(sy);
+      if (pbc & 4) sz -= nearbyintf(sz);
+      x = fh[0] * sx + fh[1] * sy + fh[2] * sz;
+      y = fh[3] * sx + fh[4] * sy + fh[5] * sz;
+      z = fh[6] * sx + fh[7] * sy + fh[8] * sz;
+    }
+  }
+};
+
 // Displacement r_j - r_i: the double difference rounded to float, then the
 // float minimum image -- the operand order of the reference's filter
 // (nep.cu:542-549), so neighbour predicates agree bit for bit.
@@ -155,6 +204,17 @@ __device__ __forceinline__ void site_delta(const Box& b, const double2& a, const
   mic_f32(b, dx, dy, dz);
 }
 
+__device__ __forceinline__ void site_delta(const MinImage& mic, const double2& a, const double2& c,
+                                           double xi, double yi, double zi, float& dx, float& dy,
+                                           float& dz, int& tj)
+{
+  dx = a.x - xi;
+  dy = a.y - yi;
+  dz = c.x - zi;
+  tj = static_cast<int>(__double_as_longlong(c.y));
+  mic(dx, dy, dz);
+}
+
 // Displacement to site j and j's type.
 __device__ __forceinline__ void site_displacement(const Box& b, const Site* __restrict__ sites,
                                                   double xi, double yi, double zi, int j,
@@ -190,6 +250,7 @@ __device__ __forceinline__ void skin_check_atom(int N, int i, const Box& b, doub
     return;
   }
   double col[3] = {0.0, 0.0, 0.0}, row_max = 0.0;
+#pragma unroll
   for (int r = 0; r < 3; ++r) {
     double row = 0.0;
     for (int c = 0; c < 3; ++c) {
@@ -199,7 +260,9 @@ __device__ __forceinline__ void skin_check_atom(int N, int i, const Box& b, doub
     }
     row_max = fmax(row_max, row);
   }
-  const double def = sqrt(fmax(fmax(col[0], col[1]), col[2]) * row_max);
+  // (no deformation since the build, the usual case: no square root)
+  const double def2 = fmax(fmax(col[0], col[1]), col[2]) * row_max;
+  const double def = def2 == 0.0 ? 0.0 : sqrt(def2);
   const double strain = fmax(fabs(1.0 - st->box_scale), def);
   const double half = 0.5 * (skin - strain * rc_v);
   if (half <= 0.0) {

@@ -256,6 +256,7 @@ __host__ __device__ constexpr int round4(int x) { return (x + 3) & ~3; }
 struct FusedLayout {
   int kpr, kpa;        // basis sizes padded to float4
   int c_rad, c_ang;    // coefficient tables [T*T][n][kp]
+  int cut_r, cut_a;    // pair cutoffs and reciprocals [T*T] float2, radial and angular
   int wt;              // transposed ANN weights [T][dim][H4], or -1: read from global
   int per_atom;        // floats of per-center scratch
   int s, a, q, fp, gh; // offsets inside one center's scratch
@@ -317,7 +318,9 @@ __host__ __device__ inline FusedLayout fused_layout(const ModelParams& p, int at
   // centers start on different banks
   L.per_atom = round4(L.gh + (tc ? 0 : p.H));
   if ((L.per_atom / 4) % 2 == 0) L.per_atom += 4;
-  const int tables = round4(L.c_ang + tt * p.nA * L.kpa);
+  L.cut_r = round4(L.c_ang + tt * p.nA * L.kpa);
+  L.cut_a = L.cut_r + 2 * tt;
+  const int tables = round4(L.cut_a + 2 * tt);
   const int wsize = p.T * p.dim * p.H4;
   L.wt = tables;
   L.atoms_base = tables + wsize;
@@ -336,23 +339,15 @@ __host__ __device__ inline FusedLayout fused_layout(const ModelParams& p, int at
   return L;
 }
 
-// Cutoff of a type pair and its reciprocal: which 0 radial, 1 angular.  The
-// exact builds read both from ModelParams::pair_cut (the correctly rounded
-// reciprocal without a division per edge); the FAST builds form them from
-// the per-type cutoffs with the hardware reciprocal, which costs less than
-// the two loads.
-template <bool FAST>
-__device__ __forceinline__ void pair_cutoff(const ModelParams& p, int which, int t1, int t2,
-                                            float& rc, float& rcinv)
+// Cutoffs of the type pairs and their correctly rounded reciprocals (computed on
+// the host, ModelParams::pair_cut) in shared memory, [T*T] of (cutoff, 1 /
+// cutoff): which 0 radial, 1 angular.  An edge reads its pair in one access.
+__device__ __forceinline__ void load_pair_cut(const ModelParams& p, int which, float2* dst)
 {
-  if constexpr (FAST) {
-    rc = which == 0 ? (p.rc_r[t1] + p.rc_r[t2]) * 0.5f : (p.rc_a[t1] + p.rc_a[t2]) * 0.5f;
-    rcinv = __fdividef(1.0f, rc);
-  } else {
-    const int tt = p.T * p.T, k = t1 * p.T + t2;
-    rc = __ldg(p.pair_cut + 2 * which * tt + k);
-    rcinv = __ldg(p.pair_cut + (2 * which + 1) * tt + k);
-  }
+  const int tt = p.T * p.T;
+  for (int k = threadIdx.x; k < tt; k += blockDim.x)
+    dst[k] = make_float2(__ldg(p.pair_cut + 2 * which * tt + k),
+                         __ldg(p.pair_cut + (2 * which + 1) * tt + k));
 }
 
 // f[k] . c[k] over KM basis values with float4 loads of a padded row, in
@@ -822,15 +817,24 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
   if constexpr (BIN == kBinShared)
     for (int q = 0; q < T * KP / 4; ++q) bin[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (blockIdx.x == 0 && tid == 0) st->rebuild = 0;   // the Verlet list is consumed
+  // per type pair: radial cutoff, its reciprocal, both cutoffs squared; then the
+  // box's matrix
+  float4* s_cut = reinterpret_cast<float4*>(
+    sm + filter_table_floats(p, KP) +
+    (BIN == kBinShared ? 4 * kBlock * filter_bin_float4(p, KP) : 0));
+  for (int k = tid; k < T * T; k += kBlock) {
+    const float rr = __ldg(p.pair_cut + k), ra = __ldg(p.pair_cut + 2 * T * T + k);
+    s_cut[k] = make_float4(rr, __ldg(p.pair_cut + T * T + k), rr * rr, ra * ra);
+  }
+  const MinImage mic(box, reinterpret_cast<float*>(s_cut + T * T));
   __syncthreads();
   const int lane = tid & 31, warp = tid >> 5;
   const int group = lane / G, gl = lane % G;
   const int i = blockIdx.x * APB + warp * APW + group;
   const bool active = i < N;
-  const Box b = *box;
   const Site me = active ? sites[i] : Site{0.0, 0.0, 0.0, 0};
   const double xi = me.x, yi = me.y, zi = me.z;
-  const int t1 = static_cast<int>(me.type);
+  const int t1 = BIN == kBinRegs ? 0 : static_cast<int>(me.type);
   const unsigned below = (1u << gl) - 1u;
   float qr[NRM];
 #pragma unroll
@@ -868,13 +872,14 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
     float x12 = 0.0f, y12 = 0.0f, z12 = 0.0f, d12_square = 0.0f, rc_radial = 1.0f;
     float rcinv_r = 1.0f;
     if (k < nv) {
-      site_delta(b, sa, sc, xi, yi, zi, x12, y12, z12, t2);
+      site_delta(mic, sa, sc, xi, yi, zi, x12, y12, z12, t2);
+      if constexpr (BIN == kBinRegs) t2 = 0;   // one type: its cutoffs stay in registers
       d12_square = x12 * x12 + y12 * y12 + z12 * z12;
-      float rc_angular, rcinv_a;
-      pair_cutoff<FAST>(p, 0, t1, t2, rc_radial, rcinv_r);
-      pair_cutoff<FAST>(p, 1, t1, t2, rc_angular, rcinv_a);
-      in_r = d12_square < rc_radial * rc_radial;
-      in_a = in_r && d12_square < rc_angular * rc_angular;
+      const float4 cut = s_cut[t1 * T + t2];
+      rc_radial = cut.x;
+      rcinv_r = cut.y;
+      in_r = d12_square < cut.z;
+      in_a = in_r && d12_square < cut.w;
     }
     const unsigned mr = group_ballot<G>(in_r, group);
     const unsigned ma = group_ballot<G>(in_a, group);
@@ -1058,7 +1063,7 @@ __device__ __forceinline__ float3 angular_edge_force(const ModelParams& p, const
 // moment derivative once for both, were no faster (1M carbon 3.35 against 3.33
 // ms, copper with its 18 edges per atom 2.40 against 2.33).
 template <int KM, int NAM, bool AG, bool FAST, bool EX>
-__device__ __forceinline__ float3 angular_edge_force4(const ModelParams& p, int t1,
+__device__ __forceinline__ float3 angular_edge_force4(const ModelParams& p, const float2* cut,
                                                      const float* ctab,
                                                      const float* __restrict__ av,
                                                      const float4& e)
@@ -1068,8 +1073,8 @@ __device__ __forceinline__ float3 angular_edge_force4(const ModelParams& p, int 
   const int nA = EX ? NAM : p.nA;
   const int nlm = EX ? NLM : (p.L_max + 1) * (p.L_max + 1) - 1;
   const int t2 = row_type(e);
-  float d, dinv, rc, rcinv, fc, fcp;
-  pair_cutoff<FAST>(p, 1, t1, t2, rc, rcinv);
+  const float rc = cut[t2].x, rcinv = cut[t2].y;
+  float d, dinv, fc, fcp;
   edge_length<FAST>(e.x * e.x + e.y * e.y + e.z * e.z, d, dinv);
   const float ux = e.x * dinv, uy = e.y * dinv, uz = e.z * dinv;
   cutoff_fc<FAST>(rc, rcinv, d, fc, fcp);
@@ -1156,11 +1161,13 @@ __device__ __forceinline__ float3 angular_edge_force4(const ModelParams& p, int 
                      SB * uz + (vz - uv * uz) * dinv);
 }
 
+// (cut: the center's type's row of the angular pair cutoffs, ctab of the tables.)
 // Forces of the edges erow[0 .. na) of one center into frow (which may be the
 // same memory: each lane reads an edge before it writes the force), by the G
 // lanes of a group, the next edge loaded one iteration early.
 template <int G, int KM, int NAM, int LMAX, bool AG, bool FAST, bool EX>
-__device__ __forceinline__ void angular_force_row(const ModelParams& p, int t1, const float* ctab,
+__device__ __forceinline__ void angular_force_row(const ModelParams& p, const float2* cut,
+                                                  const float* ctab,
                                                   const float* __restrict__ av, int na, int gl,
                                                   const float4* erow, float4* frow)
 {
@@ -1171,13 +1178,11 @@ __device__ __forceinline__ void angular_force_row(const ModelParams& p, int t1, 
     if (k + G < na) next = erow[k + G];
     float3 f;
     if constexpr (LMAX <= 4) {
-      f = angular_edge_force4<KM, NAM, AG, FAST, EX>(p, t1, ctab, av, e);
+      f = angular_edge_force4<KM, NAM, AG, FAST, EX>(p, cut, ctab, av, e);
     } else {
       const int t2 = row_type(e);
-      float rc, rcinv;
-      pair_cutoff<FAST>(p, 1, t1, t2, rc, rcinv);
       f = angular_edge_force<KM, NAM, LMAX, AG, FAST>(
-        p, ctab + t2 * p.nA * ((KM + 3) & ~3), av, rc, rcinv, e.x, e.y, e.z);
+        p, ctab + t2 * p.nA * ((KM + 3) & ~3), av, cut[t2].x, cut[t2].y, e.x, e.y, e.z);
     }
     frow[k] = make_float4(f.x, f.y, f.z, 0.0f);
   }
@@ -1240,6 +1245,10 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
     const int kk = k % Lay.kpa, row = k / Lay.kpa;
     sm[Lay.c_ang + k] = kk < kA ? __ldg(p.c_pair + p.num_c_radial + row * kA + kk) : 0.0f;
   }
+  float2* cut_r = reinterpret_cast<float2*>(sm + Lay.cut_r);
+  float2* cut_a = reinterpret_cast<float2*>(sm + Lay.cut_a);
+  load_pair_cut(p, 0, cut_r);
+  load_pair_cut(p, 1, cut_a);
   if (Lay.wt >= 0) {
     const float4* src = reinterpret_cast<const float4*>(p.w0t);
     float4* dst = reinterpret_cast<float4*>(sm + Lay.wt);
@@ -1271,8 +1280,7 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
   for (int n = 0; n < NRM; ++n) qr[n] = 0.0f;
   // q_n += sum_k c(t1,t2)[n][k] f_k(d) for one radial edge
   auto add_radial = [&](int t2, float d12_square) {
-    float rc_radial, rcinv;
-    pair_cutoff<FAST>(p, 0, t1, t2, rc_radial, rcinv);
+    const float rc_radial = cut_r[t1 * T + t2].x, rcinv = cut_r[t1 * T + t2].y;
     float d, dinv;
     edge_length<FAST>(d12_square, d, dinv);
     float fc, fcp;
@@ -1343,8 +1351,8 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
         const int t2 = row_type(e);
         float d, dinv;
         edge_length<FAST>(dx * dx + dy * dy + dz * dz, d, dinv);
-        float rc, rcinv;
-        pair_cutoff<FAST>(p, 1, t1, t2, rc, rcinv);
+        const float2 cut = cut_a[t1 * T + t2];
+        const float rc = cut.x, rcinv = cut.y;
         float fc, fcp;
         cutoff_fc<FAST>(rc, rcinv, d, fc, fcp);
         float fn[KP];
@@ -1557,14 +1565,21 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
     // place of its edge
     const float* ctab = sm + Lay.c_ang + t1 * T * nA * Lay.kpa;
     float4* frow = f12 + static_cast<size_t>(i) * mn_a;
-    angular_force_row<G, KM, NAM, LMAX, false, FAST, EX>(p, t1, ctab, s_a, na, gl, frow, frow);
+    angular_force_row<G, KM, NAM, LMAX, false, FAST, EX>(p, cut_a + t1 * T, ctab, s_a, na, gl, frow,
+                                                         frow);
   }
 }
 
-// Angular coefficient tables [T*T][nA][KP] into shared memory (zero-padded rows).
+// Angular coefficient tables [T*T][nA][KP] into shared memory (zero-padded rows),
+// and behind them the angular pair cutoffs.
+__host__ __device__ inline int angular_table_floats(const ModelParams& p, int kp)
+{
+  return p.T * p.T * (p.nA * kp + 2);
+}
 template <int KP>
 __device__ __forceinline__ void load_angular_tables(const ModelParams& p, float* sm)
 {
+  load_pair_cut(p, 1, reinterpret_cast<float2*>(sm + p.T * p.T * p.nA * KP));
   const int T = p.T, nA = p.nA, kA = p.kA;
   for (int k = threadIdx.x; k < T * T * nA * KP; k += blockDim.x) {
     const int kk = k % KP, row = k / KP;
@@ -1603,8 +1618,9 @@ k_angular_f12(const ModelParams p, int N, const Site* __restrict__ sites,
   float4* frow = f12 + static_cast<size_t>(i) * mn_a;
   // Verlet rows: k_filter_radial left the edge in the slot of its force
   const float4* erow = XR ? ea + static_cast<size_t>(i) * mn_a : frow;
-  angular_force_row<G, KM, NAM, LMAX, true, FAST, false>(p, t1, sm + t1 * T * nA * KP, ai, na, gl,
-                                                         erow, frow);
+  const float2* cut = reinterpret_cast<const float2*>(sm + T * T * nA * KP) + t1 * T;
+  angular_force_row<G, KM, NAM, LMAX, true, FAST, false>(p, cut, sm + t1 * T * nA * KP, ai, na,
+                                                         gl, erow, frow);
 }
 
 // ---------------------------------------------------------------------------
@@ -1635,15 +1651,20 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
 {
   constexpr int KP = (KM + 3) & ~3;
   extern __shared__ float sm[];
-  if constexpr (XR) {
-    load_angular_tables<KP>(p, sm);
-    __syncthreads();
-  }
+  // radial pair cutoffs, the box's matrix, (explicit rows) the angular tables
+  const int T = p.T;
+  float2* cut_r = reinterpret_cast<float2*>(sm);
+  float* s_fh = sm + 2 * T * T;
+  float* s_ang = s_fh + 18 + (2 * T * T + 18) % 4;
+  load_pair_cut(p, 0, cut_r);
+  const MinImage mic(box, s_fh);
+  if constexpr (XR) load_angular_tables<KP>(p, s_ang);
+  __syncthreads();
+  const float2* cut_a = reinterpret_cast<const float2*>(s_ang + T * T * p.nA * KP);   // XR
   const int gl = threadIdx.x % G;
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
   const bool active = i < N;
-  const Box b = *box;
-  const int T = p.T, kR = p.kR, kpr = KP;
+  const int kR = p.kR, kpr = KP;
   float F[3] = {0.0f, 0.0f, 0.0f};
   float W[9] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
   float ezbl = 0.0f;
@@ -1675,12 +1696,13 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
         dz = e.z;
       } else {
         j = jr;
-        site_displacement(b, sites, xi, yi, zi, j, dx, dy, dz, t2);
+        double2 sa, sc;
+        site_load(sites, j, sa, sc);
+        site_delta(mic, sa, sc, xi, yi, zi, dx, dy, dz, t2);
       }
       float d, dinv;
       edge_length<FAST>(dx * dx + dy * dy + dz * dz, d, dinv);
-      float rc, rcinv;
-      pair_cutoff<FAST>(p, 0, t1, t2, rc, rcinv);
+      const float rc = cut_r[t1 * T + t2].x, rcinv = cut_r[t1 * T + t2].y;
       float fc, fcp;
       cutoff_fc<FAST>(rc, rcinv, d, fc, fcp);
       float fn[KP], fnp[KP];
@@ -1757,24 +1779,25 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
           if constexpr (LMAX <= 4) {
             const float4 back =
               make_float4(-dx, -dy, -dz, __int_as_float(t1 << kRowTypeShift));
-            fij = angular_edge_force4<KM, NAM, true, FAST, false>(p, t1, sm + t1 * T * nA * KP,
-                                                                 av_i, e);
-            fji = angular_edge_force4<KM, NAM, true, FAST, false>(p, t2, sm + t2 * T * nA * KP,
-                                                                 av_j, back);
+            fij = angular_edge_force4<KM, NAM, true, FAST, false>(
+              p, cut_a + t1 * T, s_ang + t1 * T * nA * KP, av_i, e);
+            fji = angular_edge_force4<KM, NAM, true, FAST, false>(
+              p, cut_a + t2 * T, s_ang + t2 * T * nA * KP, av_j, back);
           } else {
-            float rc, rcinv;
-            pair_cutoff<FAST>(p, 1, t1, t2, rc, rcinv);
+            const float2 cut = cut_a[t1 * T + t2];
             fij = angular_edge_force<KM, NAM, LMAX, true, FAST>(
-              p, sm + (t1 * T + t2) * nA * KP, av_i, rc, rcinv, dx, dy, dz);
+              p, s_ang + (t1 * T + t2) * nA * KP, av_i, cut.x, cut.y, dx, dy, dz);
             fji = angular_edge_force<KM, NAM, LMAX, true, FAST>(
-              p, sm + (t2 * T + t1) * nA * KP, av_j, rc, rcinv, -dx, -dy, -dz);
+              p, s_ang + (t2 * T + t1) * nA * KP, av_j, cut.x, cut.y, -dx, -dy, -dz);
           }
           a12 = make_float4(fij.x, fij.y, fij.z, 0.0f);
           a21 = make_float4(fji.x, fji.y, fji.z, 0.0f);
         }
       } else {
         const int j = ja;
-        site_displacement(b, sites, xi, yi, zi, j, dx, dy, dz, t2);
+        double2 sa, sc;
+        site_load(sites, j, sa, sc);
+        site_delta(mic, sa, sc, xi, yi, zi, dx, dy, dz, t2);
         a12 = f12[static_cast<size_t>(i) * mn_a + k];
         // reverse slot: i inside j's ascending row
         const int* jrow = nl_a + static_cast<size_t>(j) * mn_a;
@@ -1918,6 +1941,15 @@ void launch_fused_t(Engine& e, int N, cudaStream_t s)
   launch_fused_tx<G, NRM, KM, NAM, XR, LMAX, MINB, TC, FF, false>(e, N, s);
 }
 
+// Dynamic shared memory above the default limit (many types): raised for the kernel.
+template <typename K>
+void allow_smem(K kernel, size_t bytes)
+{
+  if (bytes > 48 * 1024)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         static_cast<int>(bytes));
+}
+
 // The mixed precisions take the FAST builds of the filter, angular-force and
 // gather kernels (and of the descriptor kernel, whose tensor-core build is
 // FAST); they exist for the small shape, the others run the exact build.
@@ -1932,7 +1964,8 @@ void launch_filter_tf(Engine& e, int N, cudaStream_t s)
   const int blocks = (N + APB - 1) / APB;
   auto launch = [&](auto kernel, size_t bin_float4) {
     const size_t smem =
-      sizeof(float) * (filter_table_floats(p, KP) + 4 * kBlock * bin_float4);
+      sizeof(float) * (filter_table_floats(p, KP) + 4 * kBlock * bin_float4 + 4 * p.T * p.T + 20);
+    allow_smem(kernel, smem);
     kernel<<<blocks, kBlock, smem, s>>>(p, N, e.d_box, e.scratch.sites, e.d_nstate, nb.nn_v,
                                         nb.nl_v, nb.mn_v, nb.nn_r, nb.nl_r, nb.mn_r, nb.nn_a,
                                         nb.nl_a, nb.mn_a, e.scratch.f12, e.scratch.qrad);
@@ -1963,8 +1996,9 @@ void launch_f12_tf(Engine& e, int N, cudaStream_t s)
   NeighborBuffers& nb = e.nbr;
   constexpr int APB = kBlock / G;
   const int blocks = (N + APB - 1) / APB;
-  const size_t smem =
-    sizeof(float) * e.params.T * e.params.T * e.params.nA * ((KM + 3) & ~3);
+  const size_t smem = sizeof(float) * angular_table_floats(e.params, (KM + 3) & ~3);
+  allow_smem(k_angular_f12<G, KM, NAM, true, LMAX, FAST>, smem);
+  allow_smem(k_angular_f12<G, KM, NAM, false, LMAX, FAST>, smem);
   if (e.use_xr)
     k_angular_f12<G, KM, NAM, true, LMAX, FAST><<<blocks, kBlock, smem, s>>>(
       e.params, N, e.scratch.sites, nb.nn_a, nb.mn_a, e.xr.ea, e.xr.large, e.scratch.acoef,
@@ -2028,8 +2062,11 @@ void launch_gather_tf(Engine& e, int N, double* pe, double* force, double* viria
   NeighborBuffers& nb = e.nbr;
   const int threads = 256;
   const int blocks = static_cast<int>((static_cast<long long>(N) * G + threads - 1) / threads);
+  const int tt = e.params.T * e.params.T;
   const size_t smem =
-    XR ? sizeof(float) * e.params.T * e.params.T * e.params.nA * ((KM + 3) & ~3) : 0;
+    sizeof(float) * (2 * tt + 18 + (2 * tt + 18) % 4 +
+                     (XR ? angular_table_floats(e.params, (KM + 3) & ~3) : 0));
+  allow_smem(k_gather<G, KM, NAM, XR, LMAX, GMINB, FAST>, smem);
   k_gather<G, KM, NAM, XR, LMAX, GMINB, FAST><<<blocks, threads, smem, s>>>(
     e.params, N, e.d_box, e.scratch.sites, nb.nn_r, nb.nl_r, nb.mn_r, nb.nn_a, nb.nl_a, nb.mn_a,
     e.xr.er, e.xr.ea, e.scratch.acoef, e.scratch.alpha, e.scratch.f12, e.xr.large,
