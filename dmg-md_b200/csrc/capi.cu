@@ -177,9 +177,10 @@ int nepx_compute(nepx_t* h, const nepx_box* box, int n, const int* d_type, const
   const bool changed = !e.have_box || std::memcmp(&b, &e.last_box, sizeof(nepx::Box)) != 0;
   const bool rebuild = e.force_rebuild || changed || n != e.last_n;
   auto s = static_cast<cudaStream_t>(stream);
-  nepx::launch_set_box(e, b, s);
   e.box_owner = nullptr;
+  e.staged_box = &b;   // the neighbour update's launch takes the box along
   nepx::launch_neighbor_update(e, n, d_pos, d_type, rebuild, s);
+  e.staged_box = nullptr;
   if (!e.tuned) nepx::engine_autotune(e, n, d_pos, d_type, s);
   nepx::launch_force(e, n, d_pos, d_type, d_pe, d_force, d_virial,
                      (flags & NEPX_ACCUMULATE) != 0, s);

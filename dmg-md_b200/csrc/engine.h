@@ -113,6 +113,9 @@ struct Engine {
   bool have_box = false;
   bool force_rebuild = true;
   const void* box_owner = nullptr;   // md whose box the device copy holds (nullptr: none)
+  // the box of this call, while nepx_compute launches its neighbour update: that
+  // launch writes it to the device copy (in place of a launch of its own)
+  const Box* staged_box = nullptr;
   int last_n = -1;
   int group = 4;             // lanes per center in the fused kernel (autotuned)
   int fused_minb = 3;        // CTAs per SM the small-shape fused kernel is built for (autotuned)

@@ -9,10 +9,8 @@
 // displacement r12 of that image.  Rows follow (j ascending, then images
 // ia, ib, ic) and are rebuilt at every force call.
 //
-// Here one warp owns a center and its lanes take consecutive candidates j;
-// per 32-candidate chunk each lane counts its edges over all images, a warp
-// scan gives every lane its write offset and a second pass writes the edges,
-// so rows keep the reference's order.  The same kernel serves any number of
+// Here one warp owns a center and its lanes take consecutive candidates
+// (j, image) in the reference's order, compacted by ballot (ImageWalk).  The same kernel serves any number of
 // structures packed into one atom range (the batched path): a center finds
 // its structure by binary search over the structure offsets.  Structures
 // that are not small use the large-box arithmetic (double difference rounded
@@ -40,24 +38,29 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-__global__ void k_pack_sites(int N, const double* __restrict__ pos, const int* __restrict__ type,
-                             Site* __restrict__ sites, NeighborState* st)
+// The first kernel of an explicit-row evaluation: the site records, and for a
+// single system its StructInfo -- from the host when the call brings the box
+// (si_mode 2: host_si, whose box also goes to the device copy; the FP64 chain on
+// the device takes 5 us), or from the device box (1).
+__global__ void k_xr_begin(int N, const double* __restrict__ pos, const int* __restrict__ type,
+                           Site* __restrict__ sites, NeighborState* st, int si_mode,
+                           const StructInfo host_si, Box* box, double rc, StructInfo* si,
+                           int* soff)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  if (i == 0) {   // the first kernel of a force evaluation: its row maxima start here
-    st->call_nn[0] = 0;
-    st->call_nn[1] = 0;
-  }
-  sites[i] = Site{pos[i], pos[N + i], pos[2 * N + i], static_cast<long long>(type[i])};
-}
-
-// One structure spanning all N atoms, its StructInfo from the device box.
-__global__ void k_struct_from_box(const Box* __restrict__ box, double rc, int N, StructInfo* si,
-                                  int* soff, NeighborState* st)
-{
+  if (i < N)
+    sites[i] = Site{pos[i], pos[N + i], pos[2 * N + i], static_cast<long long>(type[i])};
+  if (i != 0) return;
+  st->call_nn[0] = 0;   // the row maxima of this evaluation start here
+  st->call_nn[1] = 0;
+  if (si_mode == 0) return;
   StructInfo s;
-  if (expanded_box(*box, rc, s)) st->box_error = 1;
+  if (si_mode == 2) {
+    s = host_si;
+    *box = host_si.box;
+  } else if (expanded_box(*box, rc, s)) {
+    st->box_error = 1;
+  }
   s.off = 0;
   s.n = N;
   *si = s;
@@ -99,6 +102,52 @@ __device__ __forceinline__ void small_box_delta(const StructInfo& s, float x1, f
   z12 = zj + d2 - z1;
   mic_small_box(s, x12, y12, z12);
 }
+
+// The candidates of a small-box center, (j, image) with j ascending and then the
+// images, taken 32 at a time: lane l starts at candidate l and steps by 32 in
+// the mixed radix (j, ia, ib, ic), so the hits of a ballot are in row order and
+// one sweep suffices (a lane per j counted its images' hits, scanned and swept
+// them again to write).
+struct ImageWalk {
+  int j, ia, ib, ic;          // this lane's candidate (j local to the structure)
+  int dj, da, db, dc;         // 32 candidates further
+  int nb, nc, na;
+  __device__ __forceinline__ ImageWalk(const StructInfo& s, int lane)
+  {
+    na = s.ncell[0];
+    nb = s.ncell[1];
+    nc = s.ncell[2];
+    auto split = [&](int c, int& q, int& a, int& b, int& d) {
+      d = c % nc;
+      c /= nc;
+      b = c % nb;
+      c /= nb;
+      a = c % na;
+      q = c / na;
+    };
+    split(lane, j, ia, ib, ic);
+    split(32, dj, da, db, dc);
+  }
+  __device__ __forceinline__ void next()
+  {
+    ic += dc;
+    ib += db;
+    ia += da;
+    j += dj;
+    if (ic >= nc) {
+      ic -= nc;
+      ++ib;
+    }
+    if (ib >= nb) {
+      ib -= nb;
+      ++ia;
+    }
+    if (ia >= na) {
+      ia -= na;
+      ++j;
+    }
+  }
+};
 
 __device__ __forceinline__ float4 row_entry(float x, float y, float z, int j, int t)
 {
@@ -324,49 +373,34 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
       cr = found;
       __syncwarp();   // the buffer is reused by this warp's next center
     } else if (keep) {
-      // candidates (j, image) within the cutoff plus the skin, in row order:
-      // j ascending, then the images; count per lane, scan, then write
+      // candidates (j, image) within the cutoff plus the skin, in row order
       const float x1 = pos[i], y1 = pos[total + i], z1 = pos[2 * total + i];
       int* vr = bv.vrow + static_cast<size_t>(i) * bv.mn;
+      const long long total_c =
+        static_cast<long long>(n) * (s.ncell[0] * s.ncell[1] * s.ncell[2]);
+      ImageWalk w(s, lane);
       int cv = 0;
-      for (int base = 0; base < n; base += 32) {
-        const int j = off + base + lane;
-        const bool valid = base + lane < n;
-        const float rcut = cand_cut(valid ? type[j] : 0);
-        const double xj = valid ? pos[j] : 0.0, yj = valid ? pos[total + j] : 0.0,
-                     zj = valid ? pos[2 * total + j] : 0.0;
-        const unsigned jl = static_cast<unsigned>(j - off);
-        int wv = 0;
-        for (int pass = 0; pass < 2; ++pass) {
-          int kv = 0;
-          if (valid) {
-            for (int ia = 0; ia < s.ncell[0]; ++ia)
-              for (int ib = 0; ib < s.ncell[1]; ++ib)
-                for (int ic = 0; ic < s.ncell[2]; ++ic) {
-                  if (ia == 0 && ib == 0 && ic == 0 && j == i) continue;   // self
-                  float x12, y12, z12;
-                  small_box_delta(s, x1, y1, z1, xj, yj, zj, ia, ib, ic, x12, y12, z12);
-                  if (x12 * x12 + y12 * y12 + z12 * z12 < rcut * rcut) {
-                    if (pass == 1 && wv + kv < bv.mn)
-                      vr[wv + kv] = static_cast<int>(
-                        jl | (static_cast<unsigned>(ia) << kCandIndexBits) |
-                        (static_cast<unsigned>(ib) << (kCandIndexBits + 4)) |
-                        (static_cast<unsigned>(ic) << (kCandIndexBits + 8)));
-                    ++kv;
-                  }
-                }
-          }
-          if (pass == 0) {
-            int sv = kv;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-              const int u = __shfl_up_sync(kFull, sv, o);
-              if (lane >= o) sv += u;
-            }
-            wv = cv + sv - kv;
-            cv += __shfl_sync(kFull, sv, 31);
-          }
+#pragma unroll 2
+      for (long long base = 0; base < total_c; base += 32) {
+        bool hit = false;
+        unsigned code = 0u;
+        if (w.j < n) {
+          const int j = off + w.j;
+          const float rcut = cand_cut(type[j]);
+          float x12, y12, z12;
+          small_box_delta(s, x1, y1, z1, pos[j], pos[total + j], pos[2 * total + j], w.ia, w.ib,
+                          w.ic, x12, y12, z12);
+          const bool self = j == i && w.ia == 0 && w.ib == 0 && w.ic == 0;
+          hit = !self && x12 * x12 + y12 * y12 + z12 * z12 < rcut * rcut;
+          code = static_cast<unsigned>(w.j) | (static_cast<unsigned>(w.ia) << kCandIndexBits) |
+                 (static_cast<unsigned>(w.ib) << (kCandIndexBits + 4)) |
+                 (static_cast<unsigned>(w.ic) << (kCandIndexBits + 8));
         }
+        const unsigned m = __ballot_sync(kFull, hit);
+        const int at = cv + __popc(m & below);
+        if (hit && at < bv.mn) vr[at] = static_cast<int>(code);
+        cv += __popc(m);
+        w.next();
       }
       if (lane == 0) {
         bv.vcnt[i] = min(cv, bv.mn);
@@ -380,55 +414,35 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
     } else {
       // the small-box arithmetic: float center, double image position
       const float x1 = pos[i], y1 = pos[total + i], z1 = pos[2 * total + i];
-      for (int base = 0; base < n; base += 32) {
-        const int j = off + base + lane;
-        const bool valid = base + lane < n;
-        const int t2 = valid ? type[j] : 0;
-        const float rc_radial = (rr1 + p.rc_r[t2]) * 0.5f;
-        const float rc_angular = (ra1 + p.rc_a[t2]) * 0.5f;
-        const double xj = valid ? pos[j] : 0.0, yj = valid ? pos[total + j] : 0.0,
-                     zj = valid ? pos[2 * total + j] : 0.0;
-        // pass 0 counts this lane's edges, pass 1 writes them at the scanned offsets
-        int wr = 0, wa = 0;
-        for (int pass = 0; pass < 2; ++pass) {
-          int kr = 0, ka = 0;
-          if (valid) {
-            for (int ia = 0; ia < s.ncell[0]; ++ia)
-              for (int ib = 0; ib < s.ncell[1]; ++ib)
-                for (int ic = 0; ic < s.ncell[2]; ++ic) {
-                  if (ia == 0 && ib == 0 && ic == 0 && j == i) continue;   // self
-                  float x12, y12, z12;
-                  small_box_delta(s, x1, y1, z1, xj, yj, zj, ia, ib, ic, x12, y12, z12);
-                  const float d12_square = x12 * x12 + y12 * y12 + z12 * z12;
-                  if (d12_square < rc_radial * rc_radial) {
-                    if (pass == 1 && wr + kr < mn_r)
-                      rrow[wr + kr] = row_entry(x12, y12, z12, j, t2);
-                    ++kr;
-                  }
-                  if (d12_square < rc_angular * rc_angular) {
-                    if (pass == 1 && wa + ka < mn_a)
-                      arow[wa + ka] = row_entry(x12, y12, z12, j, t2);
-                    ++ka;
-                  }
-                }
-          }
-          if (pass == 0) {
-            // exclusive warp scan of the per-lane counts
-            int sr = kr, sa = ka;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-              const int ur = __shfl_up_sync(kFull, sr, o), ua = __shfl_up_sync(kFull, sa, o);
-              if (lane >= o) {
-                sr += ur;
-                sa += ua;
-              }
-            }
-            wr = cr + sr - kr;
-            wa = ca + sa - ka;
-            cr += __shfl_sync(kFull, sr, 31);
-            ca += __shfl_sync(kFull, sa, 31);
-          }
+      const long long total_c =
+        static_cast<long long>(n) * (s.ncell[0] * s.ncell[1] * s.ncell[2]);
+      ImageWalk w(s, lane);
+#pragma unroll 2
+      for (long long base = 0; base < total_c; base += 32) {
+        bool in_r = false, in_a = false;
+        float4 entry = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (w.j < n) {
+          const int j = off + w.j;
+          const int t2 = type[j];
+          const float rc_radial = (rr1 + p.rc_r[t2]) * 0.5f;
+          const float rc_angular = (ra1 + p.rc_a[t2]) * 0.5f;
+          float x12, y12, z12;
+          small_box_delta(s, x1, y1, z1, pos[j], pos[total + j], pos[2 * total + j], w.ia, w.ib,
+                          w.ic, x12, y12, z12);
+          const float d12_square = x12 * x12 + y12 * y12 + z12 * z12;
+          const bool self = j == i && w.ia == 0 && w.ib == 0 && w.ic == 0;
+          in_r = !self && d12_square < rc_radial * rc_radial;
+          in_a = !self && d12_square < rc_angular * rc_angular;
+          entry = row_entry(x12, y12, z12, j, t2);
         }
+        const unsigned mr = __ballot_sync(kFull, in_r);
+        const unsigned ma = __ballot_sync(kFull, in_a);
+        const int at_r = cr + __popc(mr & below), at_a = ca + __popc(ma & below);
+        if (in_r && at_r < mn_r) rrow[at_r] = entry;
+        if (in_a && at_a < mn_a) arow[at_a] = entry;
+        cr += __popc(mr);
+        ca += __popc(ma);
+        w.next();
       }
     }
     if (lane == 0) {
@@ -724,13 +738,13 @@ void launch_explicit_rows(Engine& e, int N, const double* pos, const int* type,
 {
   ExplicitRows& x = e.xr;
   const int threads = 256;
-  k_pack_sites<<<(N + threads - 1) / threads, threads, 0, stream>>>(N, pos, type,
-                                                                     e.scratch.sites, e.d_nstate);
-  if (x.from_box) {
-    k_struct_from_box<<<1, 1, 0, stream>>>(e.d_box, e.model.rc_radial_max, N, x.d_si, x.d_soff,
-                                           e.d_nstate);
-    x.n_struct = 1;
-  }
+  const int si_mode = !x.from_box ? 0 : e.staged_box ? 2 : 1;
+  StructInfo host_si{};
+  if (si_mode == 2) expanded_box(*e.staged_box, e.model.rc_radial_max, host_si);
+  k_xr_begin<<<(N + threads - 1) / threads, threads, 0, stream>>>(
+    N, pos, type, e.scratch.sites, e.d_nstate, si_mode, host_si, e.d_box, e.model.rc_radial_max,
+    x.d_si, x.d_soff);
+  if (x.from_box) x.n_struct = 1;
   if (!x.from_box && x.n_cells > 0) {
     cudaMemsetAsync(x.cell_count, 0, sizeof(int) * x.n_cells, stream);
     k_xcell_assign<<<(N + threads - 1) / threads, threads, 0, stream>>>(

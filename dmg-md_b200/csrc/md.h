@@ -48,6 +48,7 @@ struct MdScalars {
   double nhc_pos[kChain], nhc_mom[kChain], nhc_mass[kChain];
   double time;         // simulated time since the segment's first step (natural units)
   unsigned long long vmax2;   // bits of max |v|^2 this step (adaptive time step; >= 0)
+  unsigned blocks_done;       // blocks of the second half kick that have left their sums
 };
 
 // Per-run constants passed by value.

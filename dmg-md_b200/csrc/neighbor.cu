@@ -157,7 +157,9 @@ __device__ __forceinline__ void warp_sort128(int (&v)[4], int p2, int lane)
 
 struct RebuildArgs {
   int N;
-  const Box* box;
+  Box* box;
+  int set_box;         // 1: host_box is the box, to be written to *box
+  Box host_box;
   const double* pos;
   const int* type;
   NeighborState* st;
@@ -205,7 +207,8 @@ k_neighbor_rebuild(const RebuildArgs a)
   const int N = a.N;
   const int tid = threadIdx.x;
   const int gtid = blockIdx.x * blockDim.x + tid, nthreads = gridDim.x * blockDim.x;
-  const Box b = *a.box;
+  const Box b = a.set_box ? a.host_box : *a.box;
+  if (a.set_box && gtid == 0) *a.box = a.host_box;   // for the launches that follow
   if (a.skin_check) {
     skin_phase(N, b, a.pos, a.type, a.x0, st, a.sites, a.skin, a.rc_v, a.force);
     grid_sync(a.gsync, st);
@@ -523,6 +526,8 @@ void launch_neighbor_update(Engine& e, int N, const double* pos, const int* type
   RebuildArgs a;
   a.N = N;
   a.box = e.d_box;
+  a.set_box = e.staged_box ? 1 : 0;
+  a.host_box = e.staged_box ? *e.staged_box : Box{};
   a.pos = pos;
   a.type = type;
   a.st = e.d_nstate;
