@@ -269,8 +269,8 @@ int nepx_neighbors(nepx_t* h, int which, int n, int* d_nn, int* d_nl, int mn, vo
   const int* nn = which == 0 ? nb.nn_r : nb.nn_a;
   const int* nl = which == 0 ? nb.nl_r : nb.nl_a;
   if (cudaMemcpyAsync(d_nn, nn, sizeof(int) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
-      cudaMemcpy2DAsync(d_nl, sizeof(int) * mn, nl, sizeof(int) * src_mn, sizeof(int) * src_mn, n,
-                        cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+      cudaMemcpy2DAsync(d_nl, sizeof(int) * mn, nl, sizeof(int) * (which == 0 ? nb.mn_r : nb.st_a),
+                        sizeof(int) * src_mn, n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return cuda_fail(h, "copy neighbour rows");
   return NEPX_OK;
 }

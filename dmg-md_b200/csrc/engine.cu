@@ -171,6 +171,8 @@ std::string engine_create(Engine& e, const std::string& nep_path, int max_atoms)
   NeighborBuffers& nb = e.nbr;
   nb.mn_r = m.MN_radial;
   nb.mn_a = m.MN_angular;
+  nb.st_a = (nb.mn_a + 7) & ~7;
+  nb.st_h = (nb.st_a / 8 + 7) & ~7;
   const double rc = m.rc_max, rv = rc + e.skin;
   nb.mn_v = static_cast<int>(m.MN_radial * rv * rv * rv / (rc * rc * rc));
   nb.mn_v = std::max(nb.mn_v, nb.mn_r);
@@ -180,11 +182,12 @@ std::string engine_create(Engine& e, const std::string& nep_path, int max_atoms)
   nb.cell_cap = std::max(N, 4096);
   bool ok = true;
   ok &= dalloc(nb.nn_v, N) == cudaSuccess;
-  ok &= dalloc(nb.nl_v, static_cast<size_t>(N) * nb.mn_v) == cudaSuccess;
+  ok &= dalloc(nb.nl_v, static_cast<size_t>(N) * std::max(nb.mn_v, 26)) == cudaSuccess;
   ok &= dalloc(nb.nn_r, N) == cudaSuccess;
   ok &= dalloc(nb.nl_r, static_cast<size_t>(N) * nb.mn_r) == cudaSuccess;
   ok &= dalloc(nb.nn_a, N) == cudaSuccess;
-  ok &= dalloc(nb.nl_a, static_cast<size_t>(N) * nb.mn_a) == cudaSuccess;
+  ok &= dalloc(nb.nl_a, static_cast<size_t>(N) * nb.st_a) == cudaSuccess;
+  ok &= dalloc(nb.heads, static_cast<size_t>(N) * nb.st_h) == cudaSuccess;
   nb.rebuild_blocks = neighbor_rebuild_blocks(nb.pow2_v);
   if (nb.rebuild_blocks < 1) return "the neighbour rebuild kernel cannot be resident on this device";
   ok &= dalloc(nb.gsync, 2) == cudaSuccess;
@@ -193,15 +196,17 @@ std::string engine_create(Engine& e, const std::string& nep_path, int max_atoms)
   ok &= dalloc(nb.cell_start, nb.cell_cap) == cudaSuccess;
   ok &= dalloc(nb.cell_atoms, N) == cudaSuccess;
   ok &= dalloc(nb.cell_of, N) == cudaSuccess;
-  ok &= dalloc(nb.cell_sites, N) == cudaSuccess;
   ok &= dalloc(nb.x0, 3 * static_cast<size_t>(N)) == cudaSuccess;
   ok &= dalloc(e.scratch.sites, N) == cudaSuccess;
   ok &= dalloc(e.scratch.qrad, static_cast<size_t>(N) * p.nR) == cudaSuccess;
-  ok &= dalloc(e.scratch.alpha, static_cast<size_t>(N) * p.T * basis_stride(p)) == cudaSuccess;
-  ok &= dalloc(e.scratch.f12, static_cast<size_t>(N) * nb.mn_a) == cudaSuccess;
+  ok &= dalloc(e.scratch.alpha, static_cast<size_t>(N) * p.T * alpha_stride(p)) == cudaSuccess;
+  ok &= dalloc(e.scratch.f12, static_cast<size_t>(N) * std::max(nb.mn_a, 2)) == cudaSuccess;
+  // the rebuild's cell-ordered site records: the forces of the last call are
+  // spent by then, and the filter after it writes the slots anew
+  nb.cell_sites = reinterpret_cast<Site*>(e.scratch.f12);
   ok &= dalloc(e.scratch.pe_ann, N) == cudaSuccess;
-  ok &= dalloc(e.scratch.acoef, static_cast<size_t>(N) * p.nA * p.nlm) == cudaSuccess;
-  ok &= dalloc(e.scratch.tune_out, 13 * static_cast<size_t>(N)) == cudaSuccess;
+  // (nl_v and acoef also hold the autotuner's throw-away outputs, 13 doubles an atom)
+  ok &= dalloc(e.scratch.acoef, static_cast<size_t>(N) * std::max(p.nA * p.nlm, 26)) == cudaSuccess;
   ok &= dalloc(e.d_box, 1) == cudaSuccess;
   ok &= dalloc(e.d_nstate, 1) == cudaSuccess;
   if (!ok) return "cudaMalloc failed (per-atom buffers)";
@@ -417,7 +422,10 @@ void engine_autotune(Engine& e, int N, const double* pos, const int* type, cudaS
     for (int k = 0; k < n_lanes; ++k) {
       e.gather_minb = gm;
       e.gather_group = gather_lanes[k];
-      double* out = e.scratch.tune_out;   // 13 N doubles: pe, force, virial
+      // 13 N doubles (pe, force, virial) in a buffer this path does not hold: the
+      // Verlet rows under explicit rows, the moment derivatives otherwise
+      double* out = e.use_xr ? reinterpret_cast<double*>(e.nbr.nl_v)
+                             : reinterpret_cast<double*>(e.scratch.acoef);
       const float t = median(5, [&] {
         launch_gather(e, N, pos, type, out, out + N, out + 4 * static_cast<size_t>(N), false,
                       stream);
@@ -531,9 +539,9 @@ void engine_destroy(Engine& e)
 {
   NeighborBuffers& nb = e.nbr;
   void* ptrs[] = {e.d_params, e.d_box, e.d_nstate, nb.nn_v, nb.nl_v, nb.nn_r, nb.nl_r,
-                  nb.nn_a, nb.nl_a, nb.gsync, nb.scan_part, nb.cell_count, nb.cell_start, nb.cell_atoms, nb.cell_of,
-                  nb.cell_sites, nb.x0, e.scratch.alpha, e.scratch.f12, e.scratch.pe_ann, e.d_w16,
-                  e.scratch.tune_out, e.scratch.acoef, e.scratch.sites, e.scratch.qrad,
+                  nb.nn_a, nb.nl_a, nb.heads, nb.gsync, nb.scan_part, nb.cell_count, nb.cell_start, nb.cell_atoms, nb.cell_of,
+                  nb.x0, e.scratch.alpha, e.scratch.f12, e.scratch.pe_ann, e.d_w16,
+                  e.scratch.acoef, e.scratch.sites, e.scratch.qrad,
                   e.xr.er, e.xr.ea, e.xr.large,
                   e.xr.d_si, e.xr.d_soff};
   for (void* q : ptrs)

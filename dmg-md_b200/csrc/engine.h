@@ -18,7 +18,9 @@ struct NeighborBuffers {
   int* nn_r = nullptr;
   int* nl_r = nullptr;   // [N][mn_r]
   int* nn_a = nullptr;
-  int* nl_a = nullptr;   // [N][mn_a]
+  int* nl_a = nullptr;   // [N][st_a], st_a = mn_a rounded up to eight
+  int* heads = nullptr;  // [N][st_h] every eighth entry of the angular rows
+  int st_a = 0, st_h = 0;
   // the cooperative rebuild kernel: its grid-barrier counters (arrivals,
   // generation), per-block partial sums of the cell scan, its block count
   unsigned* gsync = nullptr;         // [2]
@@ -29,7 +31,7 @@ struct NeighborBuffers {
   int* cell_start = nullptr;
   int* cell_atoms = nullptr;
   int* cell_of = nullptr;
-  Site* cell_sites = nullptr;   // [N] site records in cell order (beside cell_atoms)
+  Site* cell_sites = nullptr;   // [N] site records in cell order (beside cell_atoms), in f12's memory
   int cell_cap = 0;
   double* x0 = nullptr;  // positions at the last Verlet build (3N SoA)
 };
@@ -37,11 +39,10 @@ struct NeighborBuffers {
 struct ForceScratch {
   Site* sites = nullptr;     // [N] position + type records, packed by the skin check
   float* qrad = nullptr;     // [N][nR] radial descriptors from the typewise filter
-  float* alpha = nullptr;    // [N][T][kp] radial force coefficients sum_n dE/dq_n c(ti,t)[n][k]
+  float* alpha = nullptr;    // [N][T][alpha_stride] radial force coefficients sum_n dE/dq_n c(ti,t)[n][k]
   float4* f12 = nullptr;     // [N][mn_a] directed angular partial forces
   float* acoef = nullptr;    // [N][nA][24] dE/ds[n][lm] of each center
   double* pe_ann = nullptr;  // [N] site energy of the ANN
-  double* tune_out = nullptr;  // [13 N] throw-away outputs of the autotuning calls
 };
 
 // Verlet candidates of the explicit rows of a batch (the server's MD
@@ -129,8 +130,10 @@ struct Engine {
 };
 
 // Padded basis width of the kernel instance serving this model (row stride
-// of the shared-memory coefficient tables and of ForceScratch::alpha).
+// of the shared-memory coefficient tables), and the row stride of
+// ForceScratch::alpha.
 int basis_stride(const ModelParams& p);
+int alpha_stride(const ModelParams& p);
 size_t fused_smem_bytes(const ModelParams& p);
 // The same for the tensor-core (mixed-precision) build; needs the tc_* fields.
 size_t fused_tc_smem_bytes(const ModelParams& p);

@@ -32,7 +32,7 @@
 //  k_gather  radial pair force from both site energies with the per-atom
 //    alpha coefficients (w_ij = sum_k f'_k(d) alpha_i[tj][k]), the angular
 //    exchange F_i += f12(i,j) - f12(j,i) with the reverse slot found by binary
-//    search in j's sorted row (explicit rows: both directed forces evaluated
+//    search (reverse_slot) in j's sorted row (explicit rows: both directed forces evaluated
 //    here), ZBL, and the per-atom virial W_i = sum_j r_ij (x) f_ji.
 //    Reference: find_force_radial (nep.cu:756-881), gpu_find_force_many_body
 //    (potential.cu:81-210), find_force_ZBL (nep.cu:996-1111).
@@ -469,18 +469,50 @@ __device__ __forceinline__ int reduce_scatter(float* v, int gl)
   return base;
 }
 
+// Row stride of alpha: the padded basis, or for the long basis whole 32-byte
+// sectors, so that a neighbour's row is read with 32-byte loads (gather of 13,824
+// carbon atoms at basis 16: 74 -> 70 us; for the short basis's nine values they
+// cost: 1M carbon 1.19 -> 1.23 ms).
+template <int KM>
+__host__ __device__ constexpr int alpha_row() { return KM <= 9 ? round4(KM) : (KM + 7) & ~7; }
+
+// sum_k f[k] alpha[k] over KM basis values of a row of alpha in global memory.
+template <int KM>
+__device__ __forceinline__ float dot_alpha(const float* __restrict__ al, const float* f)
+{
+  if constexpr (KM <= 9) return dot_basis<KM>(al, f);
+  float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int q = 0; q + 8 <= KM; q += 8) {
+    float a[8];
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]),
+          "=f"(a[7])
+        : "l"(al + q));
+#pragma unroll
+    for (int r = 0; r < 8; r += 2)
+      acc = fma2(make_float2(a[r], a[r + 1]), make_float2(f[q + r], f[q + r + 1]), acc);
+  }
+  float sum = acc.x + acc.y;
+#pragma unroll
+  for (int k = KM & ~7; k < KM; ++k) sum = fmaf(__ldg(al + k), f[k], sum);
+  return sum;
+}
+
 // Radial force coefficients of one center, alpha[t][k] = sum_n Fp[n] c(t1,t)[n][k]
-// (the group's lanes split the T * kpr entries); c_rad: shared-memory table.
+// (the group's lanes split the T * kpr entries; rows of `row` floats); c_rad:
+// shared-memory table.
 template <int G>
 __device__ __forceinline__ void center_alpha(int T, int nR, int t1, const float* s_fp,
-                                             const float* c_rad, int kpr, int gl, float* al)
+                                             const float* c_rad, int kpr, int row, int gl,
+                                             float* al)
 {
   for (int e = gl; e < T * kpr; e += G) {
     const int t = e / kpr, kk = e % kpr;
     const float* c = c_rad + (t1 * T + t) * nR * kpr + kk;
     float acc = 0.0f;
     for (int n = 0; n < nR; ++n) acc += s_fp[n] * c[n * kpr];
-    al[e] = acc;
+    al[t * row + kk] = acc;
   }
 }
 
@@ -786,6 +818,8 @@ __device__ void tc_ann(const ModelParams& p, const FusedLayout& Lay, float* sm, 
 // carbon, descriptor stage: 3.51 ms with shared bins, 3.48 with registers).
 // Kept apart from k_nep_fused so this
 // latency-bound sweep runs at the occupancy of its own register count.
+// Every eighth entry of an angular row also goes to its row of heads, by which
+// the gather finds an entry in two loads (reverse_slot).
 // The angular edges are also written out, displacement and neighbour type, to
 // the slots their forces f12 will take: the descriptor kernel then sweeps 16
 // contiguous bytes per edge instead of fetching sites, and overwrites each
@@ -800,7 +834,8 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
                 const int* __restrict__ nn_v, const int* __restrict__ nl_v, int mn_v,
                 int* __restrict__ nn_r, int* __restrict__ nl_r, int mn_r,
                 int* __restrict__ nn_a, int* __restrict__ nl_a, int mn_a,
-                float4* __restrict__ edges, float* __restrict__ qrad)
+                int st_a, int* __restrict__ heads, int st_h, float4* __restrict__ edges,
+                float* __restrict__ qrad)
 {
   constexpr int APW = 32 / G, APB = kBlock / G;
   constexpr int KP = (KM + 3) & ~3;
@@ -846,7 +881,8 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
   const int nv_max = __reduce_max_sync(kFull, nv);
   const int* vrow = nl_v + static_cast<size_t>(i) * mn_v;
   int* rrow = nl_r + static_cast<size_t>(i) * mn_r;
-  int* arow = nl_a + static_cast<size_t>(i) * mn_a;
+  int* arow = nl_a + static_cast<size_t>(i) * st_a;
+  int* hrow = heads + static_cast<size_t>(i) * st_h;
   float4* eout = edges + static_cast<size_t>(i) * mn_a;
   int cr = 0, ca = 0;
   // the next candidate's site and the index of the one after it in flight:
@@ -920,6 +956,7 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
       const int at = ca + __popc(ma & below);
       if (at < mn_a) {
         arow[at] = j;
+        if (at % 8 == 0) hrow[at / 8] = j;
         eout[at] = make_float4(x12, y12, z12, __int_as_float(t2 << kRowTypeShift));
       }
     }
@@ -1547,8 +1584,9 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
     }
     __syncwarp();
   }
-  if (active) center_alpha<G>(T, nR, t1, s_fp, sm + Lay.c_rad, Lay.kpr, gl,
-                              alpha + static_cast<size_t>(i) * T * Lay.kpr);
+  if (active) center_alpha<G>(T, nR, t1, s_fp, sm + Lay.c_rad, Lay.kpr,
+                              alpha_row<KM>(), gl,
+                              alpha + static_cast<size_t>(i) * T * alpha_row<KM>());
   center_acoef<G, NLM>(p, nR, nA, L_max, s_s, s_a, s_fp, gl);
   __syncwarp();
 
@@ -1627,6 +1665,40 @@ k_angular_f12(const ModelParams p, int N, const Site* __restrict__ sites,
 // gather
 // ---------------------------------------------------------------------------
 
+// Eight consecutive 32-bit entries (32-byte aligned) in one load.
+__device__ __forceinline__ void load8(const int* __restrict__ at, int (&v)[8])
+{
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7])
+      : "l"(at));
+}
+
+// Slot of atom i in the ascending row of count entries, -1 if it is not there
+// (a truncated row): the last block of eight whose head is not above i, from
+// the row of heads, then the place in that block.  Two rounds of loads that each
+// wait for the one before; a binary search of a carbon row (34 entries) takes
+// six, of 11 cycles of the load pipe each, and the gather waits on them.
+__device__ __forceinline__ int reverse_slot(const int* __restrict__ row,
+                                            const int* __restrict__ heads, int count, int i)
+{
+  int block = -1;
+  for (int h0 = 0; h0 * 8 < count; h0 += 8) {
+    int v[8];
+    load8(heads + h0, v);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if ((h0 + q) * 8 < count && v[q] <= i) block = h0 + q;
+  }
+  if (block < 0) return -1;
+  int v[8], slot = -1;
+  load8(row + 8 * block, v);
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (8 * block + q < count && v[q] == i) slot = 8 * block + q;
+  return slot;
+}
+
 // XR: explicit rows.  The rows then may hold one neighbour several times
 // (periodic images), so the reverse partial force f12(j,i) is not looked up
 // but evaluated here from j's moment derivatives at -r: the angular force
@@ -1641,8 +1713,8 @@ template <int G, int KM, int NAM, bool XR, int LMAX, int GMINB, bool FAST>
 __global__ void __launch_bounds__(256, GMINB)
 k_gather(const ModelParams p, int N, const Box* __restrict__ box,
          const Site* __restrict__ sites, const int* __restrict__ nn_r, const int* __restrict__ nl_r,
-         int mn_r, const int* __restrict__ nn_a, const int* __restrict__ nl_a, int mn_a,
-         const float4* __restrict__ er, const float4* __restrict__ ea,
+         int mn_r, const int* __restrict__ nn_a, const int* __restrict__ nl_a, int mn_a, int st_a,
+         const int* __restrict__ heads, int st_h, const float4* __restrict__ er, const float4* __restrict__ ea,
          const float* __restrict__ acoef, const float* __restrict__ alpha,
          const float4* __restrict__ f12, const unsigned char* __restrict__ large,
          const double* __restrict__ pe_ann,
@@ -1664,7 +1736,8 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
   const int gl = threadIdx.x % G;
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
   const bool active = i < N;
-  const int kR = p.kR, kpr = KP;
+  const int kR = p.kR;
+  constexpr int AR = alpha_row<KM>();
   float F[3] = {0.0f, 0.0f, 0.0f};
   float W[9] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
   float ezbl = 0.0f;
@@ -1672,7 +1745,7 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
     const Site me = sites[i];
     const double xi = me.x, yi = me.y, zi = me.z;
     const int t1 = static_cast<int>(me.type);
-    const float* ali = alpha + static_cast<size_t>(i) * T * kpr;
+    const float* ali = alpha + static_cast<size_t>(i) * T * AR;
     // radial pairs: both site energies through the alpha coefficients
     const int nr = nn_r[i];
     const int* rrow = nl_r + static_cast<size_t>(i) * mn_r;
@@ -1712,8 +1785,8 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
         fnp[kk] = 0.0f;
       }
       radial_basis_d<KM>(kR, rcinv, d, fc, fcp, fn, fnp);
-      const float w12 = dot_basis<KM>(ali + t2 * kpr, fnp);
-      const float w21 = dot_basis<KM>(alpha + (static_cast<size_t>(j) * T + t1) * kpr, fnp);
+      const float w12 = dot_alpha<KM>(ali + t2 * AR, fnp);
+      const float w21 = dot_alpha<KM>(alpha + (static_cast<size_t>(j) * T + t1) * AR, fnp);
       const float s12 = w12 * dinv, s21 = w21 * dinv;
       // f12 = s12 r, f21 = -s21 r; F += f12 - f21; W += r (x) f21
       F[0] += (s12 + s21) * dx;
@@ -1726,13 +1799,14 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
       W[3] += dx * f21[1];
       W[4] += dx * f21[2];
       W[5] += dy * f21[2];
-      W[6] += dy * f21[0];
-      W[7] += dz * f21[0];
-      W[8] += dz * f21[1];
     }
+    // a radial pair force lies along its edge: its virial is symmetric
+    W[6] = W[3];
+    W[7] = W[4];
+    W[8] = W[5];
     // angular exchange and ZBL
     const int na = nn_a[i];
-    const int* arow = nl_a + static_cast<size_t>(i) * mn_a;
+    const int* arow = nl_a + static_cast<size_t>(i) * st_a;
     const bool large_i = XR && large[i];
     const int zi_ = p.Z[t1];
     const float pow_zi = p.zbl ? powf(static_cast<float>(zi_), 0.23f) : 0.0f;
@@ -1800,15 +1874,11 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
         site_delta(mic, sa, sc, xi, yi, zi, dx, dy, dz, t2);
         a12 = f12[static_cast<size_t>(i) * mn_a + k];
         // reverse slot: i inside j's ascending row
-        const int* jrow = nl_a + static_cast<size_t>(j) * mn_a;
-        const int nj = nn_a[j];
-        int lo = 0, hi = nj - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (__ldg(jrow + mid) < i) lo = mid + 1; else hi = mid;
-        }
-        a21 = f12[static_cast<size_t>(j) * mn_a + lo];
-        if (nj == 0 || __ldg(jrow + lo) != i) {
+        const int slot = reverse_slot(nl_a + static_cast<size_t>(j) * st_a,
+                                      heads + static_cast<size_t>(j) * st_h, nn_a[j], i);
+        if (slot >= 0) {
+          a21 = f12[static_cast<size_t>(j) * mn_a + slot];
+        } else {
           // only a truncated (overflowed) row can lose the reverse edge
           a21 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           atomicOr(&st->overflow, 4);
@@ -1968,7 +2038,8 @@ void launch_filter_tf(Engine& e, int N, cudaStream_t s)
     allow_smem(kernel, smem);
     kernel<<<blocks, kBlock, smem, s>>>(p, N, e.d_box, e.scratch.sites, e.d_nstate, nb.nn_v,
                                         nb.nl_v, nb.mn_v, nb.nn_r, nb.nl_r, nb.mn_r, nb.nn_a,
-                                        nb.nl_a, nb.mn_a, e.scratch.f12, e.scratch.qrad);
+                                        nb.nl_a, nb.mn_a, nb.st_a, nb.heads, nb.st_h,
+                                        e.scratch.f12, e.scratch.qrad);
   };
   const int bin = filter_bin<KM>(p);
   if (bin == kBinShared)
@@ -2069,7 +2140,7 @@ void launch_gather_tf(Engine& e, int N, double* pe, double* force, double* viria
   allow_smem(k_gather<G, KM, NAM, XR, LMAX, GMINB, FAST>, smem);
   k_gather<G, KM, NAM, XR, LMAX, GMINB, FAST><<<blocks, threads, smem, s>>>(
     e.params, N, e.d_box, e.scratch.sites, nb.nn_r, nb.nl_r, nb.mn_r, nb.nn_a, nb.nl_a, nb.mn_a,
-    e.xr.er, e.xr.ea, e.scratch.acoef, e.scratch.alpha, e.scratch.f12, e.xr.large,
+    nb.st_a, nb.heads, nb.st_h, e.xr.er, e.xr.ea, e.scratch.acoef, e.scratch.alpha, e.scratch.f12, e.xr.large,
     e.scratch.pe_ann, pe,
     force, virial, accumulate ? 1 : 0, e.d_nstate);
 }
@@ -2153,6 +2224,11 @@ void launch_gather_g(Engine& e, int N, double* pe, double* force, double* virial
 
 // Padded basis width (row stride of the coefficient tables and of alpha).
 int basis_stride(const ModelParams& p) { return small_shape(p) ? round4(kSmallK) : round4(kMaxBasis); }
+
+int alpha_stride(const ModelParams& p)
+{
+  return small_shape(p) ? alpha_row<kSmallK>() : alpha_row<kMaxBasis>();
+}
 
 bool fused_occupancy_variants(const ModelParams& p) { return small_shape(p); }
 

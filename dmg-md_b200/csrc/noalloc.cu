@@ -85,19 +85,19 @@ size_t bytes_needed(const nepx::Engine& e, int n)
   c.take<int>(N);               // nn_r
   c.take<int>(N * nb.mn_r);     // nl_r
   c.take<int>(N);               // nn_a
-  c.take<int>(N * nb.mn_a);     // nl_a
+  c.take<int>(N * nb.st_a);     // nl_a
+  c.take<int>(N * nb.st_h);     // heads
   c.take<unsigned>(2);                   // grid-barrier counters
   c.take<int>(nb.rebuild_blocks);        // cell-scan partial sums
   c.take<int>(cells);           // cell_count
   c.take<int>(cells);           // cell_start
   c.take<int>(N);               // cell_atoms
   c.take<int>(N);               // cell_of
-  c.take<nepx::Site>(N);        // cell_sites
   c.take<double>(3 * N);        // x0
   c.take<nepx::Site>(N);
   c.take<float>(N * e.params.nR);
-  c.take<float>(N * e.params.T * nepx::basis_stride(e.params));
-  c.take<float4>(N * nb.mn_a);
+  c.take<float>(N * e.params.T * nepx::alpha_stride(e.params));
+  c.take<float4>(N * std::max(nb.mn_a, 2));
   c.take<double>(N);
   c.take<float>(N * e.params.nA * e.params.nlm);
   return c.used;
@@ -189,7 +189,8 @@ extern "C" int nepx_compute_noalloc(nepx_t* h, const nepx_box* box, int n, const
     nb.nn_r = c.take<int>(N);
     nb.nl_r = c.take<int>(N * nb.mn_r);
     nb.nn_a = c.take<int>(N);
-    nb.nl_a = c.take<int>(N * nb.mn_a);
+    nb.nl_a = c.take<int>(N * nb.st_a);
+    nb.heads = c.take<int>(N * nb.st_h);
     nb.gsync = c.take<unsigned>(2);
     nb.scan_part = c.take<int>(nb.rebuild_blocks);
     nb.gsync_dirty = false;
@@ -197,13 +198,13 @@ extern "C" int nepx_compute_noalloc(nepx_t* h, const nepx_box* box, int n, const
     nb.cell_start = c.take<int>(cells);
     nb.cell_atoms = c.take<int>(N);
     nb.cell_of = c.take<int>(N);
-    nb.cell_sites = c.take<nepx::Site>(N);
     nb.x0 = c.take<double>(3 * N);
     nb.cell_cap = static_cast<int>(cells);
     e.scratch.sites = c.take<nepx::Site>(N);
     e.scratch.qrad = c.take<float>(N * e.params.nR);
-    e.scratch.alpha = c.take<float>(N * e.params.T * nepx::basis_stride(e.params));
-    e.scratch.f12 = c.take<float4>(N * nb.mn_a);
+    e.scratch.alpha = c.take<float>(N * e.params.T * nepx::alpha_stride(e.params));
+    e.scratch.f12 = c.take<float4>(N * std::max(nb.mn_a, 2));
+    nb.cell_sites = reinterpret_cast<nepx::Site*>(e.scratch.f12);   // as engine_create has it
     e.scratch.pe_ann = c.take<double>(N);
     e.scratch.acoef = c.take<float>(N * e.params.nA * e.params.nlm);
     e.capacity = n;

@@ -258,7 +258,7 @@ size_t served_bytes_per_atom(const Engine& e)
   size_t b = 16 * static_cast<size_t>(nb.mn_r + nb.mn_a);   // explicit rows (float4)
   b += 16 * static_cast<size_t>(nb.mn_a);                    // angular partial forces
   b += 2 * sizeof(int) + sizeof(Site) + 1 + 2 * sizeof(int); // counts, sites, flag, cell slots
-  b += sizeof(float) * (static_cast<size_t>(p.nA) * p.nlm + p.T * basis_stride(p) + p.nR);
+  b += sizeof(float) * (static_cast<size_t>(p.nA) * p.nlm + p.T * alpha_stride(p) + p.nR);
   b += sizeof(double);                                       // site energy
   b += 2 * (2 * sizeof(int) + 10 * sizeof(double));          // arenas: type, sid, pos, vel, mass, force
   b += 2 * (sizeof(int) * (1 + static_cast<size_t>(nb.mn_v)) + 3 * sizeof(double));   // candidates
