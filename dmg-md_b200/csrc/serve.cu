@@ -428,6 +428,7 @@ void nepx_server::run()
     int par = 0, T = 0, S = 0, t_in = 0, t_out = 0, n_cells = 0;
     double t_tick = 0.0, bytes = 0.0;
     double kept = 0.0;           // atoms of structures that keep Verlet candidates
+    bool fresh = false;          // a structure entered the arena with this step
     std::vector<Finishing> fin;
   };
   Step fly;                    // the step on the GPU
@@ -495,6 +496,13 @@ void nepx_server::run()
       }
     }
     const bool stage = !res.empty() || !adm.empty();
+    // Nothing left the arena with the last step and nothing enters it now: the
+    // structures stay where they are, with the tables the device holds.  Such a
+    // step (most of them, while MD segments run) copies no arena -- the Verlet
+    // candidates alone are a kilobyte per atom -- and uploads only what changed.
+    const bool same_set = adm.empty() && flying && fly.fin.empty() && code == NEPX_OK;
+    // the step flags are the last step's too unless it had new structures
+    const bool same_flags = same_set && !fly.fresh;
     Step nx;
     if (stage) {
       // ---- 3. stage the next step: survivors in order, then the admitted ------
@@ -566,12 +574,15 @@ void nepx_server::run()
         Resident& r = res[k];
         r.si.off = r.off;
         r.si.n = r.n;
-        h_si[par][k] = r.si;
-        h_soff[par][k] = r.off;
+        if (!same_set) {
+          h_si[par][k] = r.si;
+          h_soff[par][k] = r.off;
+          h_sdt[par][k] = r.dt / kTimeUnit;
+        }
+        nx.fresh = nx.fresh || r.fresh;
         // bit 0 steps, bit 1 keeps Verlet candidates, bit 2 builds them (new)
         c_flag[k] = (r.fresh ? 0 : 1) | (r.si.keep ? 2 : 0) | (r.fresh && r.si.keep ? 4 : 0);
         if (r.si.keep) nx.kept += r.n;
-        h_sdt[par][k] = r.dt / kTimeUnit;
         nx.bytes += static_cast<double>(r.bytes);
         const bool finishes = r.fresh ? r.md_steps == 0 : r.steps_done + 1 == r.md_steps;
         if (finishes) {
@@ -581,9 +592,13 @@ void nepx_server::run()
           nx.t_out += r.n;
         }
       }
-      h_soff[par][S] = Tn;
       c_fout[nx.fin.size()] = nx.t_out;
-      nx.n_cells = assign_cells(e, h_si[par], S);
+      if (!same_set) {
+        h_soff[par][S] = Tn;
+        nx.n_cells = assign_cells(e, h_si[par], S);
+      } else {
+        nx.n_cells = fly.n_cells;
+      }
       nx.T = Tn;
       nx.S = S;
       nx.t_in = t_in;
@@ -601,8 +616,6 @@ void nepx_server::run()
     // ---- 4. enqueue the staged step ---------------------------------------------
     if (stage) {
       const int p = nx.par;
-      Arena& A = arena[cur];
-      Arena& B = arena[1 - cur];
       int* d_src = d_ctl;
       const int* d_flag = d_ctl + 2 * MS;
       const int* d_fout = d_flag + MS;
@@ -610,23 +623,28 @@ void nepx_server::run()
       if (nx.t_in > 0)
         cudaMemcpyAsync(d_in, h_in[p], (sizeof(double) * 7 + sizeof(int)) * nx.t_in,
                         cudaMemcpyHostToDevice, s);
-      cudaMemcpyAsync(d_ctl, h_ctl[p], sizeof(int) * ctl_ints, cudaMemcpyHostToDevice, s);
-      cudaMemcpyAsync(d_sdt, h_sdt[p], sizeof(double) * nx.S, cudaMemcpyHostToDevice, s);
-      cudaMemcpyAsync(e.xr.d_si, h_si[p], sizeof(StructInfo) * nx.S, cudaMemcpyHostToDevice, s);
-      cudaMemcpyAsync(e.xr.d_soff, h_soff[p], sizeof(int) * (nx.S + 1), cudaMemcpyHostToDevice,
-                      s);
-      e.xr.n_struct = nx.S;
-      e.xr.n_cells = nx.n_cells;
-      k_arena_build<<<grid(nx.T), kThreads, 0, s>>>(
-        nx.T, nx.S, e.xr.d_soff, reinterpret_cast<const int2*>(d_src), fly_T, A.type, A.pos,
-        A.vel, A.mass, A.force, nx.t_in, d_in,
-        reinterpret_cast<const int*>(d_in + static_cast<size_t>(7) * nx.t_in), B.type, B.sid,
-        B.pos, B.vel, B.mass, B.force, A.vcnt, A.x0, B.vcnt, B.x0);
-      if (nx.kept > 0)
-        k_arena_rows<<<(nx.T + 7) / 8, kThreads, 0, s>>>(
-          nx.T, nx.S, e.xr.d_soff, reinterpret_cast<const int2*>(d_src), d_flag, B.vcnt, A.vrow,
-          B.vrow, mn_cand);
-      cur = 1 - cur;
+      if (!same_flags || !nx.fin.empty())
+        cudaMemcpyAsync(d_ctl, h_ctl[p], sizeof(int) * ctl_ints, cudaMemcpyHostToDevice, s);
+      if (!same_set) {
+        cudaMemcpyAsync(d_sdt, h_sdt[p], sizeof(double) * nx.S, cudaMemcpyHostToDevice, s);
+        cudaMemcpyAsync(e.xr.d_si, h_si[p], sizeof(StructInfo) * nx.S, cudaMemcpyHostToDevice, s);
+        cudaMemcpyAsync(e.xr.d_soff, h_soff[p], sizeof(int) * (nx.S + 1), cudaMemcpyHostToDevice,
+                        s);
+        e.xr.n_struct = nx.S;
+        e.xr.n_cells = nx.n_cells;
+        Arena& A = arena[cur];
+        Arena& B = arena[1 - cur];
+        k_arena_build<<<grid(nx.T), kThreads, 0, s>>>(
+          nx.T, nx.S, e.xr.d_soff, reinterpret_cast<const int2*>(d_src), fly_T, A.type, A.pos,
+          A.vel, A.mass, A.force, nx.t_in, d_in,
+          reinterpret_cast<const int*>(d_in + static_cast<size_t>(7) * nx.t_in), B.type, B.sid,
+          B.pos, B.vel, B.mass, B.force, A.vcnt, A.x0, B.vcnt, B.x0);
+        if (nx.kept > 0)
+          k_arena_rows<<<(nx.T + 7) / 8, kThreads, 0, s>>>(
+            nx.T, nx.S, e.xr.d_soff, reinterpret_cast<const int2*>(d_src), d_flag, B.vcnt, A.vrow,
+            B.vrow, mn_cand);
+        cur = 1 - cur;
+      }
       Arena& R = arena[cur];
       cudaMemsetAsync(d_dmax2, 0, sizeof(double) * nx.S, s);
       k_vv1_batch<<<grid(nx.T), kThreads, 0, s>>>(nx.T, R.sid, d_flag, d_sdt, e.xr.d_si, R.mass,
