@@ -43,6 +43,7 @@ struct StructInfo {
   int off, n;
   int nc[3];      // cell grid of a large structure's candidate search (nc[0] = 0: scan all atoms)
   int cell_base;  // first cell of this structure in the batch's cell arrays
+  double cell_w[3];   // widths of the cells (orthogonal boxes)
   int keep;       // 1: keeps Verlet candidates across steps (cells sized for rc + skin)
 };
 

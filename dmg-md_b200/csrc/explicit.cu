@@ -10,13 +10,13 @@
 // ia, ib, ic) and are rebuilt at every force call.
 //
 // Here one warp owns a center and its lanes take consecutive candidates
-// (j, image) in the reference's order, compacted by ballot (ImageWalk).  The same kernel serves any number of
-// structures packed into one atom range (the batched path): a center finds
-// its structure by binary search over the structure offsets.  Structures
+// (j, image) in the reference's order, compacted by ballot (ImageWalk).  The same
+// kernel serves any number of structures packed into one atom range (the batched
+// path): a center finds its structure among the structure offsets.  Structures
 // that are not small use the large-box arithmetic (double difference rounded
 // to float, float minimum image, reference nep.cu:503-561); their candidates
-// come from a cell grid of their own (cells at least rc/2 thick, 5x5x5 stencil,
-// a counting sort per batch scanned per structure), and each row is sorted
+// come from a cell grid of their own (stencil.cuh; cells at least rc/2 thick, a
+// counting sort per batch scanned per structure), and each row is sorted
 // (warp-shuffle bitonic network up to 64 entries, shared memory above), which
 // yields the large-box path's typewise rows exactly.  Those structures' rows
 // hold each neighbour once, so a batch marks their centers (large[]) for the
@@ -30,6 +30,7 @@
 #include <string>
 
 #include "engine.h"
+#include "stencil.cuh"
 #include "xbox.h"
 
 namespace nepx {
@@ -68,39 +69,65 @@ __global__ void k_xr_begin(int N, const double* __restrict__ pos, const int* __r
   soff[1] = N;
 }
 
-// Minimum image in the expanded box (reference nep_small_box.cuh:39-54).
-__device__ __forceinline__ void mic_small_box(const StructInfo& s, float& x12, float& y12,
-                                              float& z12)
-{
-  const float* e = s.eh;
-  float sx12 = e[9] * x12 + e[10] * y12 + e[11] * z12;
-  float sy12 = e[12] * x12 + e[13] * y12 + e[14] * z12;
-  float sz12 = e[15] * x12 + e[16] * y12 + e[17] * z12;
-  if (s.box.pbc[0] == 1) sx12 -= nearbyintf(sx12);
-  if (s.box.pbc[1] == 1) sy12 -= nearbyintf(sy12);
-  if (s.box.pbc[2] == 1) sz12 -= nearbyintf(sz12);
-  x12 = e[0] * sx12 + e[1] * sy12 + e[2] * sz12;
-  y12 = e[3] * sx12 + e[4] * sy12 + e[5] * sz12;
-  z12 = e[6] * sx12 + e[7] * sy12 + e[8] * sz12;
-}
+// What the small-box arithmetic reads of a structure, in registers (read through
+// the structure's pointer, every candidate loaded it again after the row writes).
+struct ImageBox {
+  float fh[9], e[18];
+  int pbc[3];
+  __device__ __forceinline__ explicit ImageBox(const StructInfo& s)
+  {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) fh[k] = s.box.fh[k];
+#pragma unroll
+    for (int k = 0; k < 18; ++k) e[k] = s.eh[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) pbc[k] = s.box.pbc[k];
+  }
+};
 
 // Displacement from a center (float position) to atom j (double position) at
 // image (ia, ib, ic) of the expanded box: the reference's small-box
-// arithmetic (nep_small_box.cuh:134-143).  Shared by the row builder and the
-// Verlet-candidate filter, so both produce the same float values.
-__device__ __forceinline__ void small_box_delta(const StructInfo& s, float x1, float y1,
-                                                float z1, double xj, double yj, double zj,
-                                                int ia, int ib, int ic, float& x12, float& y12,
-                                                float& z12)
+// arithmetic (nep_small_box.cuh:134-143) with its minimum image in the expanded
+// box (:39-54).  Shared by the row builder and the Verlet-candidate filter, so
+// both produce the same float values.
+__device__ __forceinline__ void small_box_delta(const ImageBox& s, float x1, float y1, float z1,
+                                                double xj, double yj, double zj, int ia, int ib,
+                                                int ic, float& x12, float& y12, float& z12)
 {
-  const float* fh = s.box.fh;
+  const float* fh = s.fh;
+  const float* e = s.e;
   const float d0 = fh[0] * ia + fh[1] * ib + fh[2] * ic;
   const float d1 = fh[3] * ia + fh[4] * ib + fh[5] * ic;
   const float d2 = fh[6] * ia + fh[7] * ib + fh[8] * ic;
   x12 = xj + d0 - x1;
   y12 = yj + d1 - y1;
   z12 = zj + d2 - z1;
-  mic_small_box(s, x12, y12, z12);
+  float sx12 = e[9] * x12 + e[10] * y12 + e[11] * z12;
+  float sy12 = e[12] * x12 + e[13] * y12 + e[14] * z12;
+  float sz12 = e[15] * x12 + e[16] * y12 + e[17] * z12;
+  if (s.pbc[0] == 1) sx12 -= nearbyintf(sx12);
+  if (s.pbc[1] == 1) sy12 -= nearbyintf(sy12);
+  if (s.pbc[2] == 1) sz12 -= nearbyintf(sz12);
+  x12 = e[0] * sx12 + e[1] * sy12 + e[2] * sz12;
+  y12 = e[3] * sx12 + e[4] * sy12 + e[5] * sz12;
+  z12 = e[6] * sx12 + e[7] * sy12 + e[8] * sz12;
+}
+
+// The structure of center i, the last s with soff[s] <= i, by one warp: 32
+// probes per round (two rounds up to 1,024 structures).
+__device__ __forceinline__ int warp_find_struct(const int* __restrict__ soff, int S, int i,
+                                                int lane)
+{
+  int lo = 0, n = S;
+  while (n > 1) {
+    const int step = (n + 31) >> 5;
+    const int k = lane * step;
+    const unsigned m = __ballot_sync(kFull, k < n && __ldg(soff + lo + k) <= i);
+    const int q = 31 - __clz(m);   // lane 0 always holds
+    lo += q * step;
+    n = min(step, n - q * step);
+  }
+  return lo;
 }
 
 // The candidates of a small-box center, (j, image) with j ascending and then the
@@ -154,13 +181,27 @@ __device__ __forceinline__ float4 row_entry(float x, float y, float z, int j, in
   return make_float4(x, y, z, __int_as_float(j | (t << kRowTypeShift)));
 }
 
+// The angular neighbours of large structures by index, as the Verlet path's rows
+// hold them, with every eighth in a row of heads: the gather's reverse slots.
+struct RowHeads {
+  int* nl;
+  int* heads;
+  int st_a, st_h;
+  __device__ __forceinline__ void put(int i, int at, int j) const
+  {
+    nl[static_cast<size_t>(i) * st_a + at] = j;
+    if (at % 8 == 0) heads[static_cast<size_t>(i) * st_h + at / 8] = j;
+  }
+};
+
 __global__ void __launch_bounds__(256)
 k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ si,
                 const int* __restrict__ soff, int S, const double* __restrict__ pos,
                 const int* __restrict__ type, int* __restrict__ nn_r, float4* __restrict__ er,
                 int mn_r, int* __restrict__ nn_a, float4* __restrict__ ea, int mn_a,
-                const int* __restrict__ cell_count, const int* __restrict__ cell_start,
-                const int* __restrict__ cell_atoms, const int* __restrict__ cell_of, int p2r,
+                const RowHeads rh, const int* __restrict__ cell_count, const int* __restrict__ cell_start,
+                const int* __restrict__ cell_atoms, const int* __restrict__ cell_of,
+                const Site* __restrict__ cell_sites, float rc_max, int p2r,
                 const Site* __restrict__ sites, unsigned char* __restrict__ large, int mark_large,
                 const BatchVerlet bv, NeighborState* st)
 {
@@ -169,12 +210,7 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
   const int wpb = blockDim.x >> 5;
   const unsigned below = (1u << lane) - 1u;
   for (int i = blockIdx.x * wpb + (threadIdx.x >> 5); i < total; i += gridDim.x * wpb) {
-    // structure of center i: the last s with soff[s] <= i
-    int lo = 0, hi = S - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (soff[mid] <= i) lo = mid; else hi = mid - 1;
-    }
+    const int lo = warp_find_struct(soff, S, i, lane);
     const StructInfo& s = si[lo];
     const int off = s.off, n = s.n;
     const int t1 = type[i];
@@ -195,93 +231,54 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
       const double xi = pos[i], yi = pos[total + i], zi = pos[2 * total + i];
       const Box b = s.box;   // the structure's box, held in registers for this center
       int* buf = s_rows + (threadIdx.x >> 5) * (p2r + 1);
-      int* count = buf + p2r;
-      if (lane == 0) *count = 0;
-      __syncwarp();
-      auto consider = [&](int j) {
-        // the site record: position and type in one 32-byte sector
-        float x12, y12, z12;
-        int tj;
-        site_displacement(b, sites, xi, yi, zi, j, x12, y12, z12, tj);
-        const float d12_square = x12 * x12 + y12 * y12 + z12 * z12;
-        const float rcut = keep ? cand_cut(tj) : (rr1 + p.rc_r[tj]) * 0.5f;
-        if (d12_square < rcut * rcut) {
-          const int slot = atomicAdd(count, 1);
+      int found = 0;
+      auto consider = [&](bool valid, int j, const double2& sa, const double2& sc) {
+        bool hit = false;
+        if (valid) {
+          float x12, y12, z12;
+          int tj;
+          site_delta(b, sa, sc, xi, yi, zi, x12, y12, z12, tj);
+          const float d12_square = x12 * x12 + y12 * y12 + z12 * z12;
+          const float rcut = keep ? cand_cut(tj) : (rr1 + p.rc_r[tj]) * 0.5f;
+          hit = j != i && d12_square < rcut * rcut;
+        }
+        const unsigned m = __ballot_sync(kFull, hit);
+        if (hit) {
+          const int slot = found + __popc(m & below);
           if (slot < p2r) buf[slot] = j;
         }
+        found += __popc(m);
       };
       if (s.nc[0] > 0) {
-        // the 5x5x5 cells (at least rc/2 wide) around the center's, every cell
-        // once where the grid is narrower.  In rounds of 32 stencil cells:
-        // lane q takes a cell, a warp prefix sum of the cell counts flattens
-        // their atoms into one range, and the warp sweeps that range 32
-        // candidates at a time (one cell per pass would leave most lanes idle)
-        const int nc0 = s.nc[0], nc1 = s.nc[1], nc2 = s.nc[2];
-        const int lc = cell_of[i] - s.cell_base;
-        const int cx = lc % nc0, cy = (lc / nc0) % nc1, cz = lc / (nc0 * nc1);
-        const int sp0 = (b.pbc[0] && nc0 >= 5) ? 5 : nc0;
-        const int sp1 = (b.pbc[1] && nc1 >= 5) ? 5 : nc1;
-        const int sp2 = (b.pbc[2] && nc2 >= 5) ? 5 : nc2;
-        const int ns = sp0 * sp1 * sp2;   // at most 125
-        const bool full = sp0 == 5 && sp1 == 5 && sp2 == 5;   // usual: constant divisors
-        for (int r0 = 0; r0 < ns; r0 += 32) {
-          int my_start = 0, my_cnt = 0;
-          if (r0 + lane < ns) {
-            const int q = r0 + lane;
-            int q0, q1, q2;
-            if (full) {
-              q0 = q % 5;
-              q1 = (q / 5) % 5;
-              q2 = q / 25;
-            } else {
-              q0 = q % sp0;
-              q1 = (q / sp0) % sp1;
-              q2 = q / (sp0 * sp1);
-            }
-            int gx = sp0 == 5 ? cx + q0 - 2 : q0;
-            int gy = sp1 == 5 ? cy + q1 - 2 : q1;
-            int gz = sp2 == 5 ? cz + q2 - 2 : q2;
-            if (gx < 0) gx += nc0; else if (gx >= nc0) gx -= nc0;
-            if (gy < 0) gy += nc1; else if (gy >= nc1) gy -= nc1;
-            if (gz < 0) gz += nc2; else if (gz >= nc2) gz -= nc2;
-            const int c = s.cell_base + (gz * nc1 + gy) * nc0 + gx;
-            my_start = cell_start[c];
-            my_cnt = cell_count[c];
+        // no pair cutoff of this center is above (its own + the largest) / 2, nor a
+        // candidate cutoff above the largest cutoff plus the skin
+        const double rmax = (keep ? static_cast<double>(rc_max) + bv.skin
+                                  : static_cast<double>(rr1 + rc_max) * 0.5) * (1.0 + 1e-5) + 1e-5;
+        const CellGrid grid{{s.nc[0], s.nc[1], s.nc[2]},
+                            {s.cell_w[0], s.cell_w[1], s.cell_w[2]}, s.cell_base};
+        const Stencil cand(b, grid, cell_of[i] - s.cell_base, xi, yi, zi, rmax * rmax, cell_start,
+                           cell_count, lane);
+        for (int base = 0; base < cand.total; base += 32) {
+          const int at = cand.place(base + lane);
+          const bool valid = base + lane < cand.total;
+          double2 sa = make_double2(0.0, 0.0), sc = sa;
+          int j = 0;
+          if (valid) {
+            j = cell_atoms[at];
+            site_load(cell_sites, at, sa, sc);
           }
-          int incl = my_cnt;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += v;
-          }
-          const int total_c = __shfl_sync(kFull, incl, 31);
-          for (int base = 0; base < total_c; base += 32) {
-            const int k = base + lane;
-            // stencil cell of candidate k: the first lane whose inclusive count exceeds k
-            int lo = 0;
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-              const int probe = lo + step - 1;
-              const int v = __shfl_sync(kFull, incl, probe);
-              if (v <= k) lo += step;
-            }
-            const int cstart = __shfl_sync(kFull, my_start, lo);
-            const int cincl = __shfl_sync(kFull, incl, lo);
-            const int ccnt = __shfl_sync(kFull, my_cnt, lo);
-            if (k < total_c) {
-              const int j = cell_atoms[cstart + (k - (cincl - ccnt))];
-              if (j != i) consider(j);
-            }
-          }
+          consider(valid, j, sa, sc);
         }
       } else {
         for (int base = 0; base < n; base += 32) {
           const int j = off + base + lane;
-          if (base + lane < n && j != i) consider(j);
+          const bool valid = base + lane < n;
+          double2 sa = make_double2(0.0, 0.0), sc = sa;
+          if (valid) site_load(sites, j, sa, sc);
+          consider(valid, j, sa, sc);
         }
       }
       __syncwarp();
-      const int found = *count;
       const int used = min(found, p2r);
       int p2 = 1;
       while (p2 < used) p2 <<= 1;
@@ -366,7 +363,10 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
         const unsigned ma = __ballot_sync(kFull, in_a);
         if (in_a) {
           const int at = ca + __popc(ma & below);
-          if (at < mn_a) arow[at] = entry;
+          if (at < mn_a) {
+            arow[at] = entry;
+            rh.put(i, at, __float_as_int(entry.w) & kRowIndexMask);
+          }
         }
         ca += __popc(ma);
       }
@@ -379,6 +379,7 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
       const long long total_c =
         static_cast<long long>(n) * (s.ncell[0] * s.ncell[1] * s.ncell[2]);
       ImageWalk w(s, lane);
+      const ImageBox ib(s);
       int cv = 0;
 #pragma unroll 2
       for (long long base = 0; base < total_c; base += 32) {
@@ -388,8 +389,9 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
           const int j = off + w.j;
           const float rcut = cand_cut(type[j]);
           float x12, y12, z12;
-          small_box_delta(s, x1, y1, z1, pos[j], pos[total + j], pos[2 * total + j], w.ia, w.ib,
-                          w.ic, x12, y12, z12);
+          double2 sa, sc;
+          site_load(sites, j, sa, sc);
+          small_box_delta(ib, x1, y1, z1, sa.x, sa.y, sc.x, w.ia, w.ib, w.ic, x12, y12, z12);
           const bool self = j == i && w.ia == 0 && w.ib == 0 && w.ic == 0;
           hit = !self && x12 * x12 + y12 * y12 + z12 * z12 < rcut * rcut;
           code = static_cast<unsigned>(w.j) | (static_cast<unsigned>(w.ia) << kCandIndexBits) |
@@ -417,6 +419,7 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
       const long long total_c =
         static_cast<long long>(n) * (s.ncell[0] * s.ncell[1] * s.ncell[2]);
       ImageWalk w(s, lane);
+      const ImageBox ib(s);
 #pragma unroll 2
       for (long long base = 0; base < total_c; base += 32) {
         bool in_r = false, in_a = false;
@@ -427,8 +430,9 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
           const float rc_radial = (rr1 + p.rc_r[t2]) * 0.5f;
           const float rc_angular = (ra1 + p.rc_a[t2]) * 0.5f;
           float x12, y12, z12;
-          small_box_delta(s, x1, y1, z1, pos[j], pos[total + j], pos[2 * total + j], w.ia, w.ib,
-                          w.ic, x12, y12, z12);
+          double2 sa, sc;
+          site_load(sites, j, sa, sc);
+          small_box_delta(ib, x1, y1, z1, sa.x, sa.y, sc.x, w.ia, w.ib, w.ic, x12, y12, z12);
           const float d12_square = x12 * x12 + y12 * y12 + z12 * z12;
           const bool self = j == i && w.ia == 0 && w.ib == 0 && w.ic == 0;
           in_r = !self && d12_square < rc_radial * rc_radial;
@@ -470,18 +474,14 @@ k_rows_verlet(const ModelParams p, int total, const StructInfo* __restrict__ si,
               const int* __restrict__ soff, int S, const double* __restrict__ pos,
               const int* __restrict__ type, int* __restrict__ nn_r, float4* __restrict__ er,
               int mn_r, int* __restrict__ nn_a, float4* __restrict__ ea, int mn_a,
-              const Site* __restrict__ sites, unsigned char* __restrict__ large,
+              const RowHeads rh, const Site* __restrict__ sites, unsigned char* __restrict__ large,
               const BatchVerlet bv, NeighborState* st)
 {
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   const unsigned below = (1u << lane) - 1u;
   for (int i = blockIdx.x * wpb + (threadIdx.x >> 5); i < total; i += gridDim.x * wpb) {
-    int lo = 0, hi = S - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (soff[mid] <= i) lo = mid; else hi = mid - 1;
-    }
+    const int lo = warp_find_struct(soff, S, i, lane);
     if (!(bv.sflag[lo] & 2)) continue;
     const StructInfo& s = si[lo];
     const int off = s.off;
@@ -495,6 +495,8 @@ k_rows_verlet(const ModelParams p, int total, const StructInfo* __restrict__ si,
     const double xi = pos[i], yi = pos[total + i], zi = pos[2 * total + i];
     const float x1 = static_cast<float>(xi), y1 = static_cast<float>(yi),
                 z1 = static_cast<float>(zi);
+    const Box b = s.box;
+    const ImageBox ib(s);
     for (int k0 = 0; k0 < nv; k0 += 32) {
       const int k = k0 + lane;
       bool in_r = false, in_a = false;
@@ -505,15 +507,15 @@ k_rows_verlet(const ModelParams p, int total, const StructInfo* __restrict__ si,
         float x12, y12, z12;
         if (!s.small) {
           j = off + static_cast<int>(code);
-          site_displacement(s.box, sites, xi, yi, zi, j, x12, y12, z12, t2);
+          site_displacement(b, sites, xi, yi, zi, j, x12, y12, z12, t2);
         } else {
           j = off + static_cast<int>(code & ((1u << kCandIndexBits) - 1u));
           const int ia = static_cast<int>((code >> kCandIndexBits) & 15u);
-          const int ib = static_cast<int>((code >> (kCandIndexBits + 4)) & 15u);
+          const int jb = static_cast<int>((code >> (kCandIndexBits + 4)) & 15u);
           const int ic = static_cast<int>(code >> (kCandIndexBits + 8));
           t2 = type[j];
-          small_box_delta(s, x1, y1, z1, pos[j], pos[total + j], pos[2 * total + j], ia, ib,
-                          ic, x12, y12, z12);
+          small_box_delta(ib, x1, y1, z1, pos[j], pos[total + j], pos[2 * total + j], ia, jb, ic,
+                          x12, y12, z12);
         }
         const float d12_square = x12 * x12 + y12 * y12 + z12 * z12;
         const float rc_radial = (rr1 + p.rc_r[t2]) * 0.5f;
@@ -532,7 +534,10 @@ k_rows_verlet(const ModelParams p, int total, const StructInfo* __restrict__ si,
       }
       if (in_a) {
         const int at = ca + __popc(ma & below);
-        if (at < mn_a) arow[at] = entry;
+        if (at < mn_a) {
+          arow[at] = entry;
+          if (!s.small) rh.put(i, at, __float_as_int(entry.w) & kRowIndexMask);
+        }
       }
       cr += __popc(mr);
       ca += __popc(ma);
@@ -627,14 +632,18 @@ __global__ void k_xcell_scan(const StructInfo* __restrict__ si, int* cell_count,
   }
 }
 
+// The atoms (index and site record) into their cells.
 __global__ void k_xcell_fill(int total, const int* __restrict__ cell_of, int* cell_count,
-                             const int* __restrict__ cell_start, int* cell_atoms)
+                             const int* __restrict__ cell_start, const Site* __restrict__ sites,
+                             int* cell_atoms, Site* cell_sites)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int c = cell_of[i];
   if (c < 0) return;
-  cell_atoms[cell_start[c] + atomicAdd(cell_count + c, 1)] = i;
+  const int at = cell_start[c] + atomicAdd(cell_count + c, 1);
+  cell_atoms[at] = i;
+  cell_sites[at] = sites[i];
 }
 
 __global__ void k_row_indices(int n, const int* __restrict__ cnt, const float4* __restrict__ rows,
@@ -688,7 +697,10 @@ int assign_cells(const Engine& e, StructInfo* si, int n)
     int nc[3];
     const int cells = structure_cells(e, s, nc);
     if (cells == 0 || used + cells > e.xr.cell_cap) continue;
-    for (int d = 0; d < 3; ++d) s.nc[d] = nc[d];
+    for (int d = 0; d < 3; ++d) {
+      s.nc[d] = nc[d];
+      s.cell_w[d] = s.box.h[4 * d] / nc[d];
+    }
     s.cell_base = used;
     used += cells;
   }
@@ -751,7 +763,8 @@ void launch_explicit_rows(Engine& e, int N, const double* pos, const int* type,
       N, x.d_si, x.d_soff, x.n_struct, pos, x.cell_count, x.cell_of);
     k_xcell_scan<<<x.n_struct, 1024, 0, stream>>>(x.d_si, x.cell_count, x.cell_start);
     k_xcell_fill<<<(N + threads - 1) / threads, threads, 0, stream>>>(
-      N, x.cell_of, x.cell_count, x.cell_start, x.cell_atoms);
+      N, x.cell_of, x.cell_count, x.cell_start, e.scratch.sites, x.cell_atoms,
+      e.nbr.cell_sites);
   }
   const bool verlet = !x.from_box && x.bv.sflag != nullptr;
   int p2r = 1;
@@ -760,18 +773,19 @@ void launch_explicit_rows(Engine& e, int N, const double* pos, const int* type,
   const int blocks = std::min((N + warps - 1) / warps, 148 * 8);
   const size_t smem = sizeof(int) * warps * (p2r + 1);
   BatchVerlet bv = x.bv;
+  const RowHeads rh{e.nbr.nl_a, e.nbr.heads, e.nbr.st_a, e.nbr.st_h};
   if (!verlet) bv.sflag = nullptr;
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(k_rows_explicit, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          static_cast<int>(smem));
   k_rows_explicit<<<blocks, threads, smem, stream>>>(
     e.params, N, x.d_si, x.d_soff, x.n_struct, pos, type, e.nbr.nn_r, x.er, e.nbr.mn_r,
-    e.nbr.nn_a, x.ea, e.nbr.mn_a, x.cell_count, x.cell_start, x.cell_atoms, x.cell_of, p2r,
-    e.scratch.sites, x.large, x.from_box ? 0 : 1, bv, e.d_nstate);
+    e.nbr.nn_a, x.ea, e.nbr.mn_a, rh, x.cell_count, x.cell_start, x.cell_atoms, x.cell_of, e.nbr.cell_sites,
+    e.model.rc_max, p2r, e.scratch.sites, x.large, x.from_box ? 0 : 1, bv, e.d_nstate);
   if (verlet)
     k_rows_verlet<<<blocks, threads, 0, stream>>>(
       e.params, N, x.d_si, x.d_soff, x.n_struct, pos, type, e.nbr.nn_r, x.er, e.nbr.mn_r,
-      e.nbr.nn_a, x.ea, e.nbr.mn_a, e.scratch.sites, x.large, bv, e.d_nstate);
+      e.nbr.nn_a, x.ea, e.nbr.mn_a, rh, e.scratch.sites, x.large, bv, e.d_nstate);
 }
 
 bool verlet_encodable(const StructInfo& s, double skin)

@@ -23,6 +23,7 @@
 #include <climits>
 
 #include "engine.h"
+#include "stencil.cuh"
 
 namespace nepx {
 
@@ -304,131 +305,28 @@ k_neighbor_rebuild(const RebuildArgs a)
   }
   grid_sync(a.gsync, st);
 
-  // 5. Verlet rows, one warp per center.  The 5x5x5 stencil is taken as its
-  //    25 rows of cells along x (span1 x span2 of them on narrow grids); a
-  //    row's cells are consecutive in the cell order, so its atoms are one
-  //    contiguous run of the cell-ordered arrays (two where the row wraps
-  //    around the box).  In an orthogonal box each row is trimmed to the
-  //    cells that can hold a neighbour: a row whose y-z distance from the
-  //    center exceeds rc + skin is dropped, and the x extent keeps the
-  //    offsets whose distance along x fits in what is left (the bound is the
-  //    exact geometric distance to the cell, widened by 1e-5 relative so
-  //    that no pair the float predicate accepts is ever cut).  Lane r takes
-  //    row r, a warp prefix sum of the runs flattens them into one range,
-  //    and the warp sweeps it 32 candidates at a time, reading the
-  //    cell-ordered index and site record side by side.  Hits are compacted
-  //    in order of discovery (ballot + popcount) and the row is sorted: in
-  //    registers, four values per lane, up to 128 entries; in shared memory
-  //    above.
+  // 5. Verlet rows, one warp per center (stencil.cuh); each candidate's index
+  //    and site record are read side by side.  Hits are compacted in order of
+  //    discovery (ballot + popcount) and the row is sorted: in registers, four
+  //    values per lane, up to 128 entries; in shared memory above.
   const int lane = tid & 31, warp = tid >> 5;
   const unsigned below = (1u << lane) - 1u;
   const int pow2 = a.pow2;
   int* buf = s_rows + warp * (pow2 + 1);
-  const int span0 = (b.pbc[0] && nc0 >= 5) ? 5 : nc0;
-  const int span1 = (b.pbc[1] && nc1 >= 5) ? 5 : nc1;
-  const int span2 = (b.pbc[2] && nc2 >= 5) ? 5 : nc2;
-  const int nrows = span1 * span2;   // at most 25
-  const bool prune = b.ortho != 0;
-  const double w0 = b.h[0] / nc0, w1 = b.h[4] / nc1, w2 = b.h[8] / nc2;
-  const double r2 = a.prune_square;
+  const CellGrid grid{{nc0, nc1, nc2}, {b.h[0] / nc0, b.h[4] / nc1, b.h[8] / nc2}, 0};
   for (int i = blockIdx.x * kRebuildWarps + warp; i < N; i += gridDim.x * kRebuildWarps) {
     // the site records may have been written by this launch (phase 0): plain
     // loads, which the barriers order, not the read-only path
     const double xi = a.sites[i].x, yi = a.sites[i].y, zi = a.sites[i].z;
-    const int ci = a.cell_of[i];
-    const int cx = ci % nc0, cy = (ci / nc0) % nc1, cz = ci / (nc0 * nc1);
-    int st1 = 0, n1 = 0, st2 = 0, n2 = 0;
-    if (lane < nrows) {
-      const int q1 = lane % span1, q2 = lane / span1;
-      // the center's position inside its cell, in cell widths (phase 2's
-      // fractional coordinates)
-      auto frac = [&](int d, int c, int nc) {
-        double sd = b.hinv[3 * d] * xi + b.hinv[3 * d + 1] * yi + b.hinv[3 * d + 2] * zi;
-        sd -= floor(sd);
-        return fmin(fmax(sd * nc - c, 0.0), 1.0);
-      };
-      // distance from the center to the cells k rows away along a direction
-      auto gap = [](int k, double u, double w) {
-        return k > 0 ? (k - u) * w : (k < 0 ? (u - k - 1) * w : 0.0);
-      };
-      double dyz2 = 0.0;
-      double ux = 0.0;
-      if (prune) {
-        if (span1 == 5) {
-          const double g = gap(q1 - 2, frac(1, cy, nc1), w1);
-          dyz2 += g * g;
-        }
-        if (span2 == 5) {
-          const double g = gap(q2 - 2, frac(2, cz, nc2), w2);
-          dyz2 += g * g;
-        }
-        if (span0 == 5) ux = frac(0, cx, nc0);
-      }
-      if (dyz2 < r2) {
-        int gy = span1 == 5 ? cy + q1 - 2 : q1;
-        int gz = span2 == 5 ? cz + q2 - 2 : q2;
-        if (gy < 0) gy += nc1; else if (gy >= nc1) gy -= nc1;
-        if (gz < 0) gz += nc2; else if (gz >= nc2) gz -= nc2;
-        const int row = (gz * nc1 + gy) * nc0;
-        // atoms of the row's cells c0..c1 (consecutive)
-        auto run = [&](int c0, int c1, int& st, int& n) {
-          st = a.cell_start[row + c0];
-          n = a.cell_start[row + c1] + a.cell_count[row + c1] - st;
-        };
-        if (span0 < 5) {
-          run(0, nc0 - 1, st1, n1);
-        } else {
-          int klo = -2, khi = 2;
-          if (prune) {
-            const double rx2 = r2 - dyz2;
-            auto within = [&](int k) {
-              const double g = gap(k, ux, w0);
-              return g * g < rx2;
-            };
-            klo = within(-1) ? (within(-2) ? -2 : -1) : 0;
-            khi = within(1) ? (within(2) ? 2 : 1) : 0;
-          }
-          const int g0 = cx + klo, g1 = cx + khi;
-          if (g0 < 0) {
-            run(g0 + nc0, nc0 - 1, st1, n1);
-            run(0, g1, st2, n2);
-          } else if (g1 >= nc0) {
-            run(g0, nc0 - 1, st1, n1);
-            run(0, g1 - nc0, st2, n2);
-          } else {
-            run(g0, g1, st1, n1);
-          }
-        }
-      }
-    }
-    const int my_cnt = n1 + n2;
-    int incl = my_cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    const int total_c = __shfl_sync(0xffffffffu, incl, 31);
+    const Stencil cand(b, grid, a.cell_of[i], xi, yi, zi, a.prune_square, a.cell_start,
+                       a.cell_count, lane);
     int total = 0;
-    for (int base = 0; base < total_c; base += 32) {
+    for (int base = 0; base < cand.total; base += 32) {
       const int k = base + lane;
-      // stencil row of candidate k: the first lane whose inclusive count exceeds k
-      int lo = 0;
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const int v = __shfl_sync(0xffffffffu, incl, lo + step - 1);
-        if (v <= k) lo += step;
-      }
-      const int r_incl = __shfl_sync(0xffffffffu, incl, lo);
-      const int r_cnt = __shfl_sync(0xffffffffu, my_cnt, lo);
-      const int r_st1 = __shfl_sync(0xffffffffu, st1, lo);
-      const int r_n1 = __shfl_sync(0xffffffffu, n1, lo);
-      const int r_st2 = __shfl_sync(0xffffffffu, st2, lo);
+      const int at = cand.place(k);
       bool hit = false;
       int j = 0;
-      if (k < total_c) {
-        const int local = k - (r_incl - r_cnt);
-        const int at = local < r_n1 ? r_st1 + local : r_st2 + (local - r_n1);
+      if (k < cand.total) {
         j = a.cell_atoms[at];
         double2 sa, sc;
         site_load_coherent(a.cell_sites, at, sa, sc);

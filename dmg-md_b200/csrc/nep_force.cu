@@ -1699,17 +1699,20 @@ __device__ __forceinline__ int reverse_slot(const int* __restrict__ row,
   return slot;
 }
 
-// XR: explicit rows.  The rows then may hold one neighbour several times
-// (periodic images), so the reverse partial force f12(j,i) is not looked up
-// but evaluated here from j's moment derivatives at -r: the angular force
-// work doubles and the f12 buffer and its kernel drop out.
+// ROWS: kVerlet; kImages, explicit rows that may hold one neighbour several
+// times (periodic images), so the reverse partial force f12(j,i) is not looked up
+// but evaluated here from j's moment derivatives at -r (the angular force work
+// doubles and the f12 buffer and its kernel drop out); kLarge, the explicit rows
+// of a batch's structures that are not small, which hold each neighbour once and
+// take the Verlet rows' scheme.  A batch launches both explicit builds, each over
+// its own centers: one build for both took 103 registers and two CTAs per SM for
+// the centers that need neither angular force.
 // GMINB: CTAs of 256 per SM the instance is built for (register cap), 0 for
-// none.  The Verlet-row gather comes uncapped (about 80 registers for the
-// small shape, three CTAs) and at 4 (64 registers, a few spills, a third
-// more warps); the autotuner picks one.  The small shape's explicit-row
-// FAST build is held to two CTAs (128 registers: uncapped it would take 144,
-// and one CTA per SM).
-template <int G, int KM, int NAM, bool XR, int LMAX, int GMINB, bool FAST>
+// none.  The Verlet-row gather comes uncapped (74 registers for the small shape,
+// three CTAs) and at 4 (64 registers, a third more warps); the autotuner picks
+// one.  The small shape's FAST build of kImages is held to two CTAs.
+constexpr int kVerlet = 0, kImages = 1, kLarge = 2;
+template <int G, int KM, int NAM, int ROWS, int LMAX, int GMINB, bool FAST>
 __global__ void __launch_bounds__(256, GMINB)
 k_gather(const ModelParams p, int N, const Box* __restrict__ box,
          const Site* __restrict__ sites, const int* __restrict__ nn_r, const int* __restrict__ nl_r,
@@ -1722,6 +1725,7 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
          int accumulate, NeighborState* st)
 {
   constexpr int KP = (KM + 3) & ~3;
+  constexpr bool XR = ROWS != kVerlet, IMG = ROWS == kImages;
   extern __shared__ float sm[];
   // radial pair cutoffs, the box's matrix, (explicit rows) the angular tables
   const int T = p.T;
@@ -1730,12 +1734,13 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
   float* s_ang = s_fh + 18 + (2 * T * T + 18) % 4;
   load_pair_cut(p, 0, cut_r);
   const MinImage mic(box, s_fh);
-  if constexpr (XR) load_angular_tables<KP>(p, s_ang);
+  if constexpr (IMG) load_angular_tables<KP>(p, s_ang);
   __syncthreads();
-  const float2* cut_a = reinterpret_cast<const float2*>(s_ang + T * T * p.nA * KP);   // XR
+  const float2* cut_a = reinterpret_cast<const float2*>(s_ang + T * T * p.nA * KP);   // IMG
   const int gl = threadIdx.x % G;
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const bool active = i < N;
+  bool active = i < N;
+  if constexpr (XR) active = active && (large[i] != 0) == (ROWS == kLarge);
   const int kR = p.kR;
   constexpr int AR = alpha_row<KM>();
   float F[3] = {0.0f, 0.0f, 0.0f};
@@ -1807,12 +1812,11 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
     // angular exchange and ZBL
     const int na = nn_a[i];
     const int* arow = nl_a + static_cast<size_t>(i) * st_a;
-    const bool large_i = XR && large[i];
     const int zi_ = p.Z[t1];
     const float pow_zi = p.zbl ? powf(static_cast<float>(zi_), 0.23f) : 0.0f;
     int ja_next = (!XR && gl < na) ? arow[gl] : 0;
     for (int k = gl; k < na; k += G) {
-      int t2;
+      int t2, rev;
       float dx, dy, dz;
       float4 a12, a21;
       const int ja = ja_next;
@@ -1827,24 +1831,7 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
         dx = e.x;
         dy = e.y;
         dz = e.z;
-        if (large_i) {
-          // a structure that is not small: j once in i's row and i once in
-          // j's (rows ascend by the packed index), f12 from k_angular_f12
-          a12 = f12[static_cast<size_t>(i) * mn_a + k];
-          const int* jw = reinterpret_cast<const int*>(ea + static_cast<size_t>(j) * mn_a) + 3;
-          const int nj = nn_a[j];
-          int lo = 0, hi = nj - 1;
-          while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if ((__ldg(jw + 4 * mid) & kRowIndexMask) < i) lo = mid + 1; else hi = mid;
-          }
-          a21 = f12[static_cast<size_t>(j) * mn_a + lo];
-          if (nj == 0 || (__ldg(jw + 4 * lo) & kRowIndexMask) != i) {
-            // only a truncated (overflowed) row can lose the reverse edge
-            a21 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            atomicOr(&st->overflow, 4);
-          }
-        } else {
+        if constexpr (IMG) {
           const int nA = p.nA;
           constexpr int NLM = num_lm<LMAX>();
           const float* av_i = acoef + static_cast<size_t>(i) * nA * NLM;
@@ -1867,17 +1854,20 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
           a12 = make_float4(fij.x, fij.y, fij.z, 0.0f);
           a21 = make_float4(fji.x, fji.y, fji.z, 0.0f);
         }
+        rev = j;
       } else {
-        const int j = ja;
         double2 sa, sc;
-        site_load(sites, j, sa, sc);
+        site_load(sites, ja, sa, sc);
         site_delta(mic, sa, sc, xi, yi, zi, dx, dy, dz, t2);
+        rev = ja;
+      }
+      if constexpr (!IMG) {
         a12 = f12[static_cast<size_t>(i) * mn_a + k];
         // reverse slot: i inside j's ascending row
-        const int slot = reverse_slot(nl_a + static_cast<size_t>(j) * st_a,
-                                      heads + static_cast<size_t>(j) * st_h, nn_a[j], i);
+        const int slot = reverse_slot(nl_a + static_cast<size_t>(rev) * st_a,
+                                      heads + static_cast<size_t>(rev) * st_h, nn_a[rev], i);
         if (slot >= 0) {
-          a21 = f12[static_cast<size_t>(j) * mn_a + slot];
+          a21 = f12[static_cast<size_t>(rev) * mn_a + slot];
         } else {
           // only a truncated (overflowed) row can lose the reverse edge
           a21 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -2126,7 +2116,7 @@ void set_fused_smem_wide(const ModelParams& p)
   limit(k_nep_fused<G, n, k, n, false, 4, 3, false, false, true>);
 }
 
-template <int G, int KM, int NAM, bool XR, int LMAX, int GMINB, bool FAST>
+template <int G, int KM, int NAM, int ROWS, int LMAX, int GMINB, bool FAST>
 void launch_gather_tf(Engine& e, int N, double* pe, double* force, double* virial,
                       bool accumulate, cudaStream_t s)
 {
@@ -2136,32 +2126,32 @@ void launch_gather_tf(Engine& e, int N, double* pe, double* force, double* viria
   const int tt = e.params.T * e.params.T;
   const size_t smem =
     sizeof(float) * (2 * tt + 18 + (2 * tt + 18) % 4 +
-                     (XR ? angular_table_floats(e.params, (KM + 3) & ~3) : 0));
-  allow_smem(k_gather<G, KM, NAM, XR, LMAX, GMINB, FAST>, smem);
-  k_gather<G, KM, NAM, XR, LMAX, GMINB, FAST><<<blocks, threads, smem, s>>>(
+                     (ROWS == kImages ? angular_table_floats(e.params, (KM + 3) & ~3) : 0));
+  allow_smem(k_gather<G, KM, NAM, ROWS, LMAX, GMINB, FAST>, smem);
+  k_gather<G, KM, NAM, ROWS, LMAX, GMINB, FAST><<<blocks, threads, smem, s>>>(
     e.params, N, e.d_box, e.scratch.sites, nb.nn_r, nb.nl_r, nb.mn_r, nb.nn_a, nb.nl_a, nb.mn_a,
     nb.st_a, nb.heads, nb.st_h, e.xr.er, e.xr.ea, e.scratch.acoef, e.scratch.alpha, e.scratch.f12, e.xr.large,
     e.scratch.pe_ann, pe,
     force, virial, accumulate ? 1 : 0, e.d_nstate);
 }
 
-template <int G, int KM, int NAM, bool XR, int LMAX, int GMINB = 0>
+template <int G, int KM, int NAM, int ROWS, int LMAX, int GMINB = 0>
 void launch_gather_t(Engine& e, int N, double* pe, double* force, double* virial,
                      bool accumulate, cudaStream_t s)
 {
   if constexpr (KM == kSmallK && LMAX == 4) {
     if (fast_math(e)) {
       // the FAST builds are held to their occupancy: two CTAs per SM on
-      // explicit rows, three for the uncapped Verlet-row build (it takes 84
+      // rows of images, three for the uncapped Verlet-row build (it takes 84
       // registers unheld, which the 8-register allocation unit rounds to 88:
       // two CTAs of 256, and 1.5x the time)
-      constexpr int fast_minb = XR ? 2 : (GMINB == 0 ? 3 : GMINB);
-      launch_gather_tf<G, KM, NAM, XR, LMAX, fast_minb, true>(e, N, pe, force, virial,
-                                                              accumulate, s);
+      constexpr int fast_minb = ROWS == kImages ? 2 : (GMINB == 0 ? 3 : GMINB);
+      launch_gather_tf<G, KM, NAM, ROWS, LMAX, fast_minb, true>(e, N, pe, force, virial,
+                                                                accumulate, s);
       return;
     }
   }
-  launch_gather_tf<G, KM, NAM, XR, LMAX, GMINB, false>(e, N, pe, force, virial, accumulate, s);
+  launch_gather_tf<G, KM, NAM, ROWS, LMAX, GMINB, false>(e, N, pe, force, virial, accumulate, s);
 }
 
 // the FP32 build or, for the mixed precisions, the tensor-core one
@@ -2212,10 +2202,16 @@ template <int G, int KM, int NAM, int LMAX>
 void launch_gather_g(Engine& e, int N, double* pe, double* force, double* virial,
                      bool accumulate, cudaStream_t s)
 {
-  if (e.use_xr) launch_gather_t<G, KM, NAM, true, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
-  else if (LMAX == 4 && e.gather_minb == 4)
-    launch_gather_t<G, KM, NAM, false, LMAX, 4>(e, N, pe, force, virial, accumulate, s);
-  else launch_gather_t<G, KM, NAM, false, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
+  if (e.use_xr) {
+    launch_gather_t<G, KM, NAM, kImages, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
+    if (e.xr.from_box) return;
+    if (LMAX == 4) launch_gather_t<G, KM, NAM, kLarge, LMAX, 4>(e, N, pe, force, virial, accumulate, s);
+    else launch_gather_t<G, KM, NAM, kLarge, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
+  } else if (LMAX == 4 && e.gather_minb == 4) {
+    launch_gather_t<G, KM, NAM, kVerlet, LMAX, 4>(e, N, pe, force, virial, accumulate, s);
+  } else {
+    launch_gather_t<G, KM, NAM, kVerlet, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
+  }
 }
 
 }  // namespace
