@@ -115,9 +115,18 @@ struct MinImage {
   // Called by every thread of the block, with a barrier before the first use;
   // s_fh: 18 floats of shared memory.
   __device__ __forceinline__ MinImage(const Box* __restrict__ b, float* s_fh)
+    : MinImage(*b, static_cast<const float*>(s_fh))
   {
     for (int k = threadIdx.x; k < 18; k += blockDim.x) s_fh[k] = b->fh[k];
-    fh = s_fh;
+  }
+
+  // The matrix read where it is (a warp with a box of its own).
+  __device__ __forceinline__ explicit MinImage(const Box& b) : MinImage(b, b.fh) {}
+
+  __device__ __forceinline__ MinImage(const Box& box, const float* matrix)
+  {
+    const Box* b = &box;
+    fh = matrix;
     lx = b->fh[0];
     ly = b->fh[4];
     lz = b->fh[8];

@@ -67,6 +67,11 @@ struct BatchVerlet {
 constexpr int kCandIndexBits = 20;
 constexpr int kCandMaxImages = 16;
 
+// Kinds of structures (ExplicitRows::kinds): those with the small-box image
+// arithmetic, and the others.  Each has its own row, angular-force and gather
+// launches, left out where there is none.
+constexpr int kSmallRows = 1, kLargeRows = 2;
+
 // Explicit-row state: the small-box path (one structure, rebuilt from the
 // device box at every call) and the batched path (many structures).
 struct ExplicitRows {
@@ -77,6 +82,7 @@ struct ExplicitRows {
   int max_struct = 0;
   int n_struct = 0;
   bool from_box = true;       // one structure whose StructInfo follows the device box
+  int kinds = kSmallRows | kLargeRows;   // what the structures are, or may be
   // cell lists of the large structures of a batch (candidate search)
   int* cell_count = nullptr;
   int* cell_start = nullptr;
@@ -201,8 +207,8 @@ std::string engine_enable_xr(Engine& e, int max_struct);
 // Cell grids of the large structures of a batch: each gets cells at least
 // rc / 2 thick, (rc + skin) / 2 where it keeps Verlet candidates (at most
 // cell_cap in total, else it scans all its atoms); returns the number of
-// cells.  Structures are described by si[0..n).
-int assign_cells(const Engine& e, StructInfo* si, int n);
+// cells.  Structures are described by si[0..n), whose kinds it records in e.xr.
+int assign_cells(Engine& e, StructInfo* si, int n);
 // Cells of a structure's grid (0: small, or too few cells for the stencil,
 // so its rows scan all its atoms); nc_out (may be null) gets the grid.
 int structure_cells(const Engine& e, const StructInfo& s, int* nc_out);

@@ -194,7 +194,12 @@ struct RowHeads {
   }
 };
 
-__global__ void __launch_bounds__(256)
+// Rows of the centers of small structures (SMALL: images), or of the others. One
+// kernel for both took 97 registers, two CTAs per SM, and issued on 46 % of its
+// cycles; apart, and held to three and four CTAs, they took the batch call of 188
+// structures from 2.54 to 2.21 ms.
+template <bool SMALL>
+__global__ void __launch_bounds__(256, SMALL ? 3 : 4)
 k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ si,
                 const int* __restrict__ soff, int S, const double* __restrict__ pos,
                 const int* __restrict__ type, int* __restrict__ nn_r, float4* __restrict__ er,
@@ -212,6 +217,7 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
   for (int i = blockIdx.x * wpb + (threadIdx.x >> 5); i < total; i += gridDim.x * wpb) {
     const int lo = warp_find_struct(soff, S, i, lane);
     const StructInfo& s = si[lo];
+    if ((s.small != 0) != SMALL) continue;
     const int off = s.off, n = s.n;
     const int t1 = type[i];
     const float rr1 = p.rc_r[t1], ra1 = p.rc_a[t1];
@@ -227,9 +233,9 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
     float4* rrow = er + static_cast<size_t>(i) * mn_r;
     float4* arow = ea + static_cast<size_t>(i) * mn_a;
     int cr = 0, ca = 0;
-    if (!s.small) {
+    if constexpr (!SMALL) {
       const double xi = pos[i], yi = pos[total + i], zi = pos[2 * total + i];
-      const Box b = s.box;   // the structure's box, held in registers for this center
+      const MinImage mic(s.box);
       int* buf = s_rows + (threadIdx.x >> 5) * (p2r + 1);
       int found = 0;
       auto consider = [&](bool valid, int j, const double2& sa, const double2& sc) {
@@ -237,7 +243,7 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
         if (valid) {
           float x12, y12, z12;
           int tj;
-          site_delta(b, sa, sc, xi, yi, zi, x12, y12, z12, tj);
+          site_delta(mic, sa, sc, xi, yi, zi, x12, y12, z12, tj);
           const float d12_square = x12 * x12 + y12 * y12 + z12 * z12;
           const float rcut = keep ? cand_cut(tj) : (rr1 + p.rc_r[tj]) * 0.5f;
           hit = j != i && d12_square < rcut * rcut;
@@ -256,7 +262,7 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
                                   : static_cast<double>(rr1 + rc_max) * 0.5) * (1.0 + 1e-5) + 1e-5;
         const CellGrid grid{{s.nc[0], s.nc[1], s.nc[2]},
                             {s.cell_w[0], s.cell_w[1], s.cell_w[2]}, s.cell_base};
-        const Stencil cand(b, grid, cell_of[i] - s.cell_base, xi, yi, zi, rmax * rmax, cell_start,
+        const Stencil cand(s.box, grid, cell_of[i] - s.cell_base, xi, yi, zi, rmax * rmax, cell_start,
                            cell_count, lane);
         for (int base = 0; base < cand.total; base += 32) {
           const int at = cand.place(base + lane);
@@ -353,7 +359,9 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
           const int j = buf[k];
           float x12, y12, z12;
           int t2;
-          site_displacement(b, sites, xi, yi, zi, j, x12, y12, z12, t2);
+          double2 sa, sc;
+          site_load(sites, j, sa, sc);
+          site_delta(mic, sa, sc, xi, yi, zi, x12, y12, z12, t2);
           const float d12_square = x12 * x12 + y12 * y12 + z12 * z12;
           const float rc_angular = (ra1 + p.rc_a[t2]) * 0.5f;
           in_a = d12_square < rc_angular * rc_angular;
@@ -452,7 +460,7 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
     if (lane == 0) {
       nn_r[i] = min(cr, mn_r);
       nn_a[i] = min(ca, mn_a);
-      large[i] = mark_large && !s.small ? 1 : 0;
+      large[i] = mark_large && !SMALL ? 1 : 0;
       if (cr > mn_r) atomicOr(&st->overflow, 2);
       if (ca > mn_a) atomicOr(&st->overflow, 4);
       atomicMax(&st->max_nn[1], cr);
@@ -469,7 +477,7 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
 // bit while no atom of the structure has moved more than skin / 2 since the
 // candidates were built.  Radial and angular rows are written in order by
 // warp ballot + popcount.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 k_rows_verlet(const ModelParams p, int total, const StructInfo* __restrict__ si,
               const int* __restrict__ soff, int S, const double* __restrict__ pos,
               const int* __restrict__ type, int* __restrict__ nn_r, float4* __restrict__ er,
@@ -495,7 +503,7 @@ k_rows_verlet(const ModelParams p, int total, const StructInfo* __restrict__ si,
     const double xi = pos[i], yi = pos[total + i], zi = pos[2 * total + i];
     const float x1 = static_cast<float>(xi), y1 = static_cast<float>(yi),
                 z1 = static_cast<float>(zi);
-    const Box b = s.box;
+    const MinImage mic(s.box);
     const ImageBox ib(s);
     for (int k0 = 0; k0 < nv; k0 += 32) {
       const int k = k0 + lane;
@@ -507,7 +515,9 @@ k_rows_verlet(const ModelParams p, int total, const StructInfo* __restrict__ si,
         float x12, y12, z12;
         if (!s.small) {
           j = off + static_cast<int>(code);
-          site_displacement(b, sites, xi, yi, zi, j, x12, y12, z12, t2);
+          double2 sa, sc;
+          site_load(sites, j, sa, sc);
+          site_delta(mic, sa, sc, xi, yi, zi, x12, y12, z12, t2);
         } else {
           j = off + static_cast<int>(code & ((1u << kCandIndexBits) - 1u));
           const int ia = static_cast<int>((code >> kCandIndexBits) & 15u);
@@ -687,11 +697,13 @@ int structure_cells(const Engine& e, const StructInfo& s, int* nc_out)
   return cells;
 }
 
-int assign_cells(const Engine& e, StructInfo* si, int n)
+int assign_cells(Engine& e, StructInfo* si, int n)
 {
   int used = 0;
+  e.xr.kinds = 0;
   for (int k = 0; k < n; ++k) {
     StructInfo& s = si[k];
+    e.xr.kinds |= s.small ? kSmallRows : kLargeRows;
     s.nc[0] = s.nc[1] = s.nc[2] = 0;
     s.cell_base = 0;
     int nc[3];
@@ -756,7 +768,11 @@ void launch_explicit_rows(Engine& e, int N, const double* pos, const int* type,
   k_xr_begin<<<(N + threads - 1) / threads, threads, 0, stream>>>(
     N, pos, type, e.scratch.sites, e.d_nstate, si_mode, host_si, e.d_box, e.model.rc_radial_max,
     x.d_si, x.d_soff);
-  if (x.from_box) x.n_struct = 1;
+  if (x.from_box) {
+    x.n_struct = 1;
+    // the box's kind where the host knows it (MD under a barostat does not)
+    x.kinds = si_mode != 2 ? kSmallRows | kLargeRows : host_si.small ? kSmallRows : kLargeRows;
+  }
   if (!x.from_box && x.n_cells > 0) {
     cudaMemsetAsync(x.cell_count, 0, sizeof(int) * x.n_cells, stream);
     k_xcell_assign<<<(N + threads - 1) / threads, threads, 0, stream>>>(
@@ -775,13 +791,18 @@ void launch_explicit_rows(Engine& e, int N, const double* pos, const int* type,
   BatchVerlet bv = x.bv;
   const RowHeads rh{e.nbr.nl_a, e.nbr.heads, e.nbr.st_a, e.nbr.st_h};
   if (!verlet) bv.sflag = nullptr;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_rows_explicit, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(smem));
-  k_rows_explicit<<<blocks, threads, smem, stream>>>(
-    e.params, N, x.d_si, x.d_soff, x.n_struct, pos, type, e.nbr.nn_r, x.er, e.nbr.mn_r,
-    e.nbr.nn_a, x.ea, e.nbr.mn_a, rh, x.cell_count, x.cell_start, x.cell_atoms, x.cell_of, e.nbr.cell_sites,
-    e.model.rc_max, p2r, e.scratch.sites, x.large, x.from_box ? 0 : 1, bv, e.d_nstate);
+  auto rows = [&](auto kernel, size_t bytes) {
+    if (bytes > 48 * 1024)
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(bytes));
+    kernel<<<blocks, threads, bytes, stream>>>(
+      e.params, N, x.d_si, x.d_soff, x.n_struct, pos, type, e.nbr.nn_r, x.er, e.nbr.mn_r,
+      e.nbr.nn_a, x.ea, e.nbr.mn_a, rh, x.cell_count, x.cell_start, x.cell_atoms, x.cell_of,
+      e.nbr.cell_sites, e.model.rc_max, p2r, e.scratch.sites, x.large, x.from_box ? 0 : 1, bv,
+      e.d_nstate);
+  };
+  if (x.kinds & kSmallRows) rows(k_rows_explicit<true>, 0);
+  if (x.kinds & kLargeRows) rows(k_rows_explicit<false>, smem);
   if (verlet)
     k_rows_verlet<<<blocks, threads, 0, stream>>>(
       e.params, N, x.d_si, x.d_soff, x.n_struct, pos, type, e.nbr.nn_r, x.er, e.nbr.mn_r,

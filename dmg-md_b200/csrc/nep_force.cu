@@ -2203,8 +2203,10 @@ void launch_gather_g(Engine& e, int N, double* pe, double* force, double* virial
                      bool accumulate, cudaStream_t s)
 {
   if (e.use_xr) {
-    launch_gather_t<G, KM, NAM, kImages, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
-    if (e.xr.from_box) return;
+    // a single system takes the images' scheme whatever its box
+    if (e.xr.from_box || (e.xr.kinds & kSmallRows))
+      launch_gather_t<G, KM, NAM, kImages, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
+    if (e.xr.from_box || !(e.xr.kinds & kLargeRows)) return;
     if (LMAX == 4) launch_gather_t<G, KM, NAM, kLarge, LMAX, 4>(e, N, pe, force, virial, accumulate, s);
     else launch_gather_t<G, KM, NAM, kLarge, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
   } else if (LMAX == 4 && e.gather_minb == 4) {
@@ -2320,7 +2322,7 @@ void launch_descriptor(Engine& e, int N, const double*, const int*, cudaStream_t
   }
   // a single explicit-row system: the gather evaluates both directed angular
   // forces itself; a batch's structures that are not small take f12 here
-  if (e.use_xr && e.xr.from_box) return;
+  if (e.use_xr && (e.xr.from_box || !(e.xr.kinds & kLargeRows))) return;
   if (fused_angular_force(e)) return;   // the descriptor kernel wrote f12
   if (high) launch_f12_t<kHighGroup, kMaxBasis, kMaxN, 8>(e, N, stream);
   else if (e.f12_group >= 8) {
