@@ -8,12 +8,12 @@
 // filters it into typewise radial and angular lists with float
 // d^2 < ((rc_t1 + rc_t2)/2)^2.  Rows are ascending in atom index.
 //
-// B200 design: everything stays on the device, in one cooperative launch.
-// Its phases -- skin check, cell grid, counting sort of the atoms into cells,
-// Verlet rows -- are separated by grid-wide barriers (every
-// block is resident, and every wait is bounded); a step whose skin check
-// finds nothing to rebuild costs that one launch, which returns at once, and
-// never waits on the host.  Rows are row-major (atom i owns the contiguous
+// B200 design: everything stays on the device.  The skin check is a plain kernel
+// (in an MD step, part of the first half kick); the rebuild is one cooperative
+// launch whose phases -- cell grid, counting sort of the atoms into cells, Verlet
+// rows -- are separated by grid-wide barriers (every block is resident, and every
+// wait is bounded).  A step with nothing to rebuild costs that launch, which
+// returns at once, and never waits on the host.  Rows are row-major (atom i owns the contiguous
 // slots [i*MN, i*MN + count)) so the warp that owns a center reads and writes
 // coalesced.  The cell list is a counting sort on a grid of cells at least
 // (rc + skin)/2 wide with a 5x5x5 stencil; each Verlet row is sorted in
@@ -29,7 +29,10 @@ namespace nepx {
 
 namespace {
 
-constexpr int kRebuildThreads = 128;                 // four warps: a center per warp in the row build
+// Sixteen warps, a center per warp in the row build: CTAs of four warps hold the
+// same number, but four times the arrivals at every barrier.
+constexpr int kRebuildThreads = 512;
+constexpr int kRebuildCtas = 3;                      // per SM (42 registers)
 constexpr int kRebuildWarps = kRebuildThreads / 32;
 constexpr long long kGridWaitCycles = 4000000000ll;  // ~2 s at the B200 clock
 
@@ -42,17 +45,25 @@ __device__ __forceinline__ int wrapped_cell(double s, int nc, int pbc)
 }
 
 // Packs each atom into its Site record for the neighbour sweeps of this
-// step and applies the skin criterion (skin_check_atom, common.cuh).  The MD
-// step does the same inside its first half kick instead.
-__device__ __forceinline__ void skin_phase(int N, const Box& b, const double* __restrict__ pos,
-                                           const int* __restrict__ type,
-                                           const double* __restrict__ x0, NeighborState* st,
-                                           Site* __restrict__ sites, double skin, double rc_v,
-                                           int force)
+// step and applies the skin criterion (skin_check_atom, common.cuh); the MD
+// step does the same inside its first half kick instead.  The call's box, when it
+// brings one, goes to the device copy here.  (As the first phase of the
+// cooperative rebuild it put a grid-wide barrier on every call: neighbour stage
+// of 24,000 atoms 19 us, of 1,551 atoms 11 us.)
+__global__ void __launch_bounds__(256)
+k_skin(int N, Box* box, int set_box, const Box host_box, const double* __restrict__ pos,
+       const int* __restrict__ type, const double* __restrict__ x0, NeighborState* st,
+       Site* __restrict__ sites, double skin, double rc_v, int force)
 {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
-    skin_check_atom(N, i, b, pos[i], pos[N + i], pos[2 * N + i], type[i], x0, st, sites, skin,
-                    rc_v, force);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (set_box && i == 0) *box = host_box;   // for the launches that follow
+  if (i >= N) return;
+  const Box* b = box;
+  Box mine;
+  if (set_box) mine = host_box;
+  else mine = *b;
+  skin_check_atom(N, i, mine, pos[i], pos[N + i], pos[2 * N + i], type[i], x0, st, sites, skin,
+                  rc_v, force);
 }
 
 // Grid-wide barrier of the cooperative rebuild.  A generation counter: the
@@ -158,9 +169,7 @@ __device__ __forceinline__ void warp_sort128(int (&v)[4], int p2, int lane)
 
 struct RebuildArgs {
   int N;
-  Box* box;
-  int set_box;         // 1: host_box is the box, to be written to *box
-  Box host_box;
+  const Box* box;
   const double* pos;
   const int* type;
   NeighborState* st;
@@ -176,16 +185,13 @@ struct RebuildArgs {
   unsigned* gsync;
   int* part;           // [gridDim.x] per-block sums of the cell scan
   int mn_v, pow2, cell_cap;
-  double skin, rc_v;
+  double rc_v;
   float cutoff_square;
   double prune_square; // (rc_v (1 + 1e-5) + 1e-5)^2: the stencil rows' trimming bound
-  int skin_check;      // 1: pack the sites and apply the skin criterion first
-  int force;           // with skin_check: rebuild whatever the displacements
 };
 
-// The whole neighbour update in one cooperative launch (grid-stride phases,
-// grid_sync between them):
-//   0. (skin_check) site records and the skin criterion;
+// The rebuild of the Verlet rows in one cooperative launch (grid-stride phases,
+// grid_sync between them), after the site records and the skin criterion:
 //   1. cell grid from the current box (cells at least rc_v/2 thick, at most
 //      cell_cap of them), counts cleared;
 //   2. cell of every atom, counts;
@@ -196,9 +202,9 @@ struct RebuildArgs {
 //      d^2 < (rc + skin)^2, sorts the row (bitonic, in registers up to 128
 //      entries) and writes it with the reference positions of the next skin
 //      check.
-// Phases 1-5 run only when the rebuild flag is set; the flag is the same for
-// every block, so all of them return together.
-__global__ void __launch_bounds__(kRebuildThreads, 12)
+// They run only when the rebuild flag is set; the flag is the same for every
+// block, so all of them return together.
+__global__ void __launch_bounds__(kRebuildThreads, kRebuildCtas)
 k_neighbor_rebuild(const RebuildArgs a)
 {
   extern __shared__ int s_rows[];
@@ -208,13 +214,8 @@ k_neighbor_rebuild(const RebuildArgs a)
   const int N = a.N;
   const int tid = threadIdx.x;
   const int gtid = blockIdx.x * blockDim.x + tid, nthreads = gridDim.x * blockDim.x;
-  const Box b = a.set_box ? a.host_box : *a.box;
-  if (a.set_box && gtid == 0) *a.box = a.host_box;   // for the launches that follow
-  if (a.skin_check) {
-    skin_phase(N, b, a.pos, a.type, a.x0, st, a.sites, a.skin, a.rc_v, a.force);
-    grid_sync(a.gsync, st);
-  }
-  if (!*reinterpret_cast<volatile int*>(&st->rebuild)) return;
+  if (!st->rebuild) return;
+  const Box b = *a.box;
 
   // 1. cell grid (every block derives the same one; block 0 records it)
   if (tid == 0) {
@@ -315,8 +316,6 @@ k_neighbor_rebuild(const RebuildArgs a)
   int* buf = s_rows + warp * (pow2 + 1);
   const CellGrid grid{{nc0, nc1, nc2}, {b.h[0] / nc0, b.h[4] / nc1, b.h[8] / nc2}, 0};
   for (int i = blockIdx.x * kRebuildWarps + warp; i < N; i += gridDim.x * kRebuildWarps) {
-    // the site records may have been written by this launch (phase 0): plain
-    // loads, which the barriers order, not the read-only path
     const double xi = a.sites[i].x, yi = a.sites[i].y, zi = a.sites[i].z;
     const Stencil cand(b, grid, a.cell_of[i], xi, yi, zi, a.prune_square, a.cell_start,
                        a.cell_count, lane);
@@ -400,7 +399,10 @@ size_t rebuild_smem(int pow2) { return sizeof(int) * kRebuildWarps * (pow2 + 1);
 int neighbor_rebuild_blocks(int pow2_v)
 {
   int dev = 0, sms = 0, per_sm = 0;
+  // long rows' sort buffers exceed the default limit (rows are capped at 2,048)
   if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaFuncSetAttribute(k_neighbor_rebuild, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(rebuild_smem(2048))) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_neighbor_rebuild, kRebuildThreads,
                                                     rebuild_smem(pow2_v)) != cudaSuccess)
@@ -424,8 +426,6 @@ void launch_neighbor_update(Engine& e, int N, const double* pos, const int* type
   RebuildArgs a;
   a.N = N;
   a.box = e.d_box;
-  a.set_box = e.staged_box ? 1 : 0;
-  a.host_box = e.staged_box ? *e.staged_box : Box{};
   a.pos = pos;
   a.type = type;
   a.st = e.d_nstate;
@@ -443,13 +443,15 @@ void launch_neighbor_update(Engine& e, int N, const double* pos, const int* type
   a.mn_v = nb.mn_v;
   a.pow2 = nb.pow2_v;
   a.cell_cap = nb.cell_cap;
-  a.skin = e.skin;
   a.rc_v = static_cast<double>(e.model.rc_max) + e.skin;
   a.cutoff_square = static_cast<float>(a.rc_v * a.rc_v);
   const double rp = a.rc_v * (1.0 + 1e-5) + 1e-5;
   a.prune_square = rp * rp;
-  a.skin_check = skin_done ? 0 : 1;
-  a.force = force ? 1 : 0;
+  if (!skin_done)
+    k_skin<<<(N + 255) / 256, 256, 0, stream>>>(N, e.d_box, e.staged_box ? 1 : 0,
+                                                e.staged_box ? *e.staged_box : Box{}, pos, type,
+                                                nb.x0, e.d_nstate, e.scratch.sites, e.skin, a.rc_v,
+                                                force ? 1 : 0);
   // small systems take fewer blocks: cheaper barriers, nothing to share out
   const int want = std::max(1, (N + kRebuildWarps - 1) / kRebuildWarps);
   cudaLaunchConfig_t cfg = {};
