@@ -172,7 +172,7 @@ std::string engine_create(Engine& e, const std::string& nep_path, int max_atoms)
   nb.mn_r = m.MN_radial;
   nb.mn_a = m.MN_angular;
   nb.st_a = (nb.mn_a + 7) & ~7;
-  nb.st_h = (nb.st_a / 8 + 7) & ~7;
+  nb.st_h = (1 + nb.st_a / 8 + 7) & ~7;
   const double rc = m.rc_max, rv = rc + e.skin;
   nb.mn_v = static_cast<int>(m.MN_radial * rv * rv * rv / (rc * rc * rc));
   nb.mn_v = std::max(nb.mn_v, nb.mn_r);

@@ -19,7 +19,7 @@ struct NeighborBuffers {
   int* nl_r = nullptr;   // [N][mn_r]
   int* nn_a = nullptr;
   int* nl_a = nullptr;   // [N][st_a], st_a = mn_a rounded up to eight
-  int* heads = nullptr;  // [N][st_h] every eighth entry of the angular rows
+  int* heads = nullptr;  // [N][st_h] length and every eighth entry of the angular rows
   int st_a = 0, st_h = 0;
   // the cooperative rebuild kernel: its grid-barrier counters (arrivals,
   // generation), per-block partial sums of the cell scan, its block count

@@ -182,7 +182,8 @@ __device__ __forceinline__ float4 row_entry(float x, float y, float z, int j, in
 }
 
 // The angular neighbours of large structures by index, as the Verlet path's rows
-// hold them, with every eighth in a row of heads: the gather's reverse slots.
+// hold them, with the length and every eighth in a row of heads: the gather's
+// reverse slots.
 struct RowHeads {
   int* nl;
   int* heads;
@@ -190,7 +191,11 @@ struct RowHeads {
   __device__ __forceinline__ void put(int i, int at, int j) const
   {
     nl[static_cast<size_t>(i) * st_a + at] = j;
-    if (at % 8 == 0) heads[static_cast<size_t>(i) * st_h + at / 8] = j;
+    if (at % 8 == 0) heads[static_cast<size_t>(i) * st_h + 1 + at / 8] = j;
+  }
+  __device__ __forceinline__ void length(int i, int n) const
+  {
+    heads[static_cast<size_t>(i) * st_h] = n;
   }
 };
 
@@ -460,6 +465,7 @@ k_rows_explicit(const ModelParams p, int total, const StructInfo* __restrict__ s
     if (lane == 0) {
       nn_r[i] = min(cr, mn_r);
       nn_a[i] = min(ca, mn_a);
+      if constexpr (!SMALL) rh.length(i, min(ca, mn_a));
       large[i] = mark_large && !SMALL ? 1 : 0;
       if (cr > mn_r) atomicOr(&st->overflow, 2);
       if (ca > mn_a) atomicOr(&st->overflow, 4);
@@ -555,6 +561,7 @@ k_rows_verlet(const ModelParams p, int total, const StructInfo* __restrict__ si,
     if (lane == 0) {
       nn_r[i] = min(cr, mn_r);
       nn_a[i] = min(ca, mn_a);
+      if (!s.small) rh.length(i, min(ca, mn_a));
       large[i] = s.small ? 0 : 1;
       if (cr > mn_r) atomicOr(&st->overflow, 2);
       if (ca > mn_a) atomicOr(&st->overflow, 4);

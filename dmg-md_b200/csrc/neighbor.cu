@@ -139,32 +139,47 @@ __device__ __forceinline__ void cx_pair(int& lo, int& hi, bool ascending)
   hi = ascending ? c : a;
 }
 
-// Ascending bitonic sort of the first p2 (a power of two, at most 128)
-// values of a warp, four per lane: element e = lane + 32 r is v[r] (padding
-// INT_MAX).  Partners e ^ jj exchange by shuffle (jj < 32) or inside the
-// lane (jj = 32, 64); e keeps the smaller value when (e < partner) matches the
-// ascending direction (e & k) == 0 of its block.
-__device__ __forceinline__ void warp_sort128(int (&v)[4], int p2, int lane)
+// Ascending bitonic sort of the first p2 (a power of two, at most 32 R) values
+// of a warp, R per lane: element e = lane + 32 r is v[r] (padding INT_MAX).
+// Partners e ^ jj exchange by shuffle (jj < 32) or inside the lane (jj >= 32);
+// e keeps the smaller value when (e < partner) matches the ascending direction
+// (e & k) == 0 of its block.
+template <int R>
+__device__ __forceinline__ void warp_sort(int (&v)[R], int p2, int lane)
 {
   for (int k = 2; k <= p2; k <<= 1) {
-    for (int jj = k >> 1; jj > 0; jj >>= 1) {
-      if (jj == 64) {
-        cx_pair(v[0], v[2], (lane & k) == 0);
-        cx_pair(v[1], v[3], ((lane + 32) & k) == 0);
-      } else if (jj == 32) {
-        cx_pair(v[0], v[1], (lane & k) == 0);
-        cx_pair(v[2], v[3], ((lane + 64) & k) == 0);
-      } else {
-        const bool lower = (lane & jj) == 0;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int pv = __shfl_xor_sync(0xffffffffu, v[r], jj);
-          const bool asc = ((lane + 32 * r) & k) == 0;
-          v[r] = (lower == asc) ? min(v[r], pv) : max(v[r], pv);
-        }
+    for (int step = R / 2; step > 0; step >>= 1) {
+      if (32 * step <= (k >> 1)) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if ((r & step) == 0) cx_pair(v[r], v[r + step], ((lane + 32 * r) & k) == 0);
+      }
+    }
+    for (int jj = min(16, k >> 1); jj > 0; jj >>= 1) {
+      const bool lower = (lane & jj) == 0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int pv = __shfl_xor_sync(0xffffffffu, v[r], jj);
+        const bool asc = ((lane + 32 * r) & k) == 0;
+        v[r] = (lower == asc) ? min(v[r], pv) : max(v[r], pv);
       }
     }
   }
+}
+
+// Sorts the used first entries of buf in registers and writes keep of them.
+template <int R>
+__device__ __forceinline__ void sort_row(const int* buf, int used, int p2, int keep, int* row,
+                                         int lane)
+{
+  int v[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = lane + 32 * r < used ? buf[lane + 32 * r] : INT_MAX;
+  warp_sort(v, p2, lane);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (lane + 32 * r < keep) row[lane + 32 * r] = v[r];
 }
 
 struct RebuildArgs {
@@ -308,8 +323,8 @@ k_neighbor_rebuild(const RebuildArgs a)
 
   // 5. Verlet rows, one warp per center (stencil.cuh); each candidate's index
   //    and site record are read side by side.  Hits are compacted in order of
-  //    discovery (ballot + popcount) and the row is sorted: in registers, four
-  //    values per lane, up to 128 entries; in shared memory above.
+  //    discovery (ballot + popcount) and the row is sorted: in registers up to
+  //    256 entries, in shared memory above.
   const int lane = tid & 31, warp = tid >> 5;
   const unsigned below = (1u << lane) - 1u;
   const int pow2 = a.pow2;
@@ -349,13 +364,11 @@ k_neighbor_rebuild(const RebuildArgs a)
     const int keep = min(total, a.mn_v);
     int* row = a.nl_v + static_cast<size_t>(i) * a.mn_v;
     if (p2 <= 128) {
-      int v[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) v[r] = lane + 32 * r < used ? buf[lane + 32 * r] : INT_MAX;
-      warp_sort128(v, p2, lane);
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-        if (lane + 32 * r < keep) row[lane + 32 * r] = v[r];
+      sort_row<4>(buf, used, p2, keep, row, lane);
+    } else if (p2 == 256) {
+      // (in shared memory: 36 passes of four pairs per lane; the rebuild of 24,000
+      // water atoms, whose rows hold 144, 271 -> 171 us)
+      sort_row<8>(buf, used, p2, keep, row, lane);
     } else {
       // bitonic sort of the smallest power of two that holds the row (padding
       // INT_MAX), one compare-exchange pair per lane and pass

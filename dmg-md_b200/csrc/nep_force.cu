@@ -818,8 +818,8 @@ __device__ void tc_ann(const ModelParams& p, const FusedLayout& Lay, float* sm, 
 // carbon, descriptor stage: 3.51 ms with shared bins, 3.48 with registers).
 // Kept apart from k_nep_fused so this
 // latency-bound sweep runs at the occupancy of its own register count.
-// Every eighth entry of an angular row also goes to its row of heads, by which
-// the gather finds an entry in two loads (reverse_slot).
+// The length of an angular row and its every eighth entry also go to its row of
+// heads, by which the gather finds an entry in two loads (reverse_slot).
 // The angular edges are also written out, displacement and neighbour type, to
 // the slots their forces f12 will take: the descriptor kernel then sweeps 16
 // contiguous bytes per edge instead of fetching sites, and overwrites each
@@ -956,7 +956,7 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
       const int at = ca + __popc(ma & below);
       if (at < mn_a) {
         arow[at] = j;
-        if (at % 8 == 0) hrow[at / 8] = j;
+        if (at % 8 == 0) hrow[1 + at / 8] = j;
         eout[at] = make_float4(x12, y12, z12, __int_as_float(t2 << kRowTypeShift));
       }
     }
@@ -981,6 +981,7 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
   if (active && gl == 0) {
     nn_r[i] = min(cr, mn_r);
     nn_a[i] = min(ca, mn_a);
+    hrow[0] = min(ca, mn_a);
     if (cr > mn_r) atomicOr(&st->overflow, 2);
     if (ca > mn_a) atomicOr(&st->overflow, 4);
     atomicMax(&st->max_nn[1], cr);
@@ -1674,24 +1675,30 @@ __device__ __forceinline__ void load8(const int* __restrict__ at, int (&v)[8])
       : "l"(at));
 }
 
-// Slot of atom i in the ascending row of count entries, -1 if it is not there
-// (a truncated row): the last block of eight whose head is not above i, from
-// the row of heads, then the place in that block.  Two rounds of loads that each
-// wait for the one before; a binary search of a carbon row (34 entries) takes
-// six, of 11 cycles of the load pipe each, and the gather waits on them.
+// Slot of atom i in an ascending row, -1 if it is not there (a truncated row):
+// the last block of eight whose head is not above i, from the row of heads (the
+// row's length, then its every eighth entry), then the place in that block.  Two
+// rounds of loads that each wait for the one before; a binary search of a carbon
+// row (34 entries) takes seven with the length, of 11 cycles of the load pipe each,
+// and the gather is bound by that pipe (75 % busy).
 __device__ __forceinline__ int reverse_slot(const int* __restrict__ row,
-                                            const int* __restrict__ heads, int count, int i)
+                                            const int* __restrict__ heads, int i)
 {
+  int v[8];
+  load8(heads, v);
+  const int count = v[0];
   int block = -1;
-  for (int h0 = 0; h0 * 8 < count; h0 += 8) {
-    int v[8];
+#pragma unroll
+  for (int q = 1; q < 8; ++q)
+    if (8 * (q - 1) < count && v[q] <= i) block = q - 1;
+  for (int h0 = 8; 8 * (h0 - 1) < count; h0 += 8) {   // rows above 56 entries
     load8(heads + h0, v);
 #pragma unroll
     for (int q = 0; q < 8; ++q)
-      if ((h0 + q) * 8 < count && v[q] <= i) block = h0 + q;
+      if (8 * (h0 + q - 1) < count && v[q] <= i) block = h0 + q - 1;
   }
   if (block < 0) return -1;
-  int v[8], slot = -1;
+  int slot = -1;
   load8(row + 8 * block, v);
 #pragma unroll
   for (int q = 0; q < 8; ++q)
@@ -1865,7 +1872,7 @@ k_gather(const ModelParams p, int N, const Box* __restrict__ box,
         a12 = f12[static_cast<size_t>(i) * mn_a + k];
         // reverse slot: i inside j's ascending row
         const int slot = reverse_slot(nl_a + static_cast<size_t>(rev) * st_a,
-                                      heads + static_cast<size_t>(rev) * st_h, nn_a[rev], i);
+                                      heads + static_cast<size_t>(rev) * st_h, i);
         if (slot >= 0) {
           a21 = f12[static_cast<size_t>(rev) * mn_a + slot];
         } else {
