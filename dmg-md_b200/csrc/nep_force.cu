@@ -1267,7 +1267,8 @@ k_nep_fused(const ModelParams p, int N, const Site* __restrict__ sites, Neighbor
   constexpr int KP = (KM + 3) & ~3;
   constexpr int NLM = num_lm<LMAX>();
   // radial functions per moment sweep
-  constexpr int CN = LMAX <= 4 ? (MINB >= 4 ? kChunkN4 : kChunkN) : 1;
+  constexpr int CN =
+    LMAX <= 4 ? (MINB >= (KM <= 9 ? 4 : 3) ? kChunkN4 : kChunkN) : 1;
   extern __shared__ __align__(128) float sm[];
   const FusedLayout Lay = fused_layout(p, APB, KP, fused_smem_budget(MINB), TC);
   const int tid = threadIdx.x;
@@ -2175,6 +2176,28 @@ void launch_fused_g(Engine& e, int N, cudaStream_t s)
   }
 }
 
+// the general shape at 2 CTAs per SM (five n per moment sweep) or, with
+// Engine::fused_minb 4, at 3 (three n): FP32; the tensor-core build comes at 2
+// (13,824 carbon atoms at n_max 12 8, basis 16 12: 238 registers and 208 us of
+// descriptor stage against 164 and 201; with the angular force inside 187)
+template <int G>
+void launch_fused_general(Engine& e, int N, cudaStream_t s)
+{
+  constexpr int n = kMaxN, k = kMaxBasis;
+  if (!e.use_xr && e.fuse_f12) {
+    if (e.precision != 0) launch_fused_t<G, n, k, n, false, 4, 2, true, true>(e, N, s);
+    else if (e.fused_minb == 4) launch_fused_t<G, n, k, n, false, 4, 3, false, true>(e, N, s);
+    else launch_fused_t<G, n, k, n, false, 4, 2, false, true>(e, N, s);
+    return;
+  }
+  if (e.fused_minb == 4 && e.precision == 0) {
+    if (e.use_xr) launch_fused_t<G, n, k, n, true, 4, 3, false>(e, N, s);
+    else launch_fused_t<G, n, k, n, false, 4, 3, false>(e, N, s);
+  } else {
+    launch_fused_g<G, n, k, n, 4, 2>(e, N, s);
+  }
+}
+
 // the small shape at 3 or 4 CTAs per SM (Engine::fused_minb, autotuned; the
 // tensor-core build comes at 3)
 template <int G>
@@ -2235,7 +2258,7 @@ int alpha_stride(const ModelParams& p)
   return small_shape(p) ? alpha_row<kSmallK>() : alpha_row<kMaxBasis>();
 }
 
-bool fused_occupancy_variants(const ModelParams& p) { return small_shape(p); }
+bool fused_occupancy_variants(const ModelParams& p) { return !high_degree(p); }
 
 bool fused_wide_groups(const Engine& e) { return exact_shape(e.params) && e.precision == 0; }
 
@@ -2272,11 +2295,13 @@ void set_fused_smem_limits(const ModelParams& p)
       set_fused_smem_t<8, kSmallN, kSmallK, kSmallN, 4, 3, true, true>(p);
     }
   } else {
-    set_fused_smem_t<4, kMaxN, kMaxBasis, kMaxN, 4, 2, false>(p);
-    set_fused_smem_t<8, kMaxN, kMaxBasis, kMaxN, 4, 2, false>(p);
+    set_fused_smem_t<4, kMaxN, kMaxBasis, kMaxN, 4, 2, false, true>(p);
+    set_fused_smem_t<8, kMaxN, kMaxBasis, kMaxN, 4, 2, false, true>(p);
+    set_fused_smem_t<4, kMaxN, kMaxBasis, kMaxN, 4, 3, false, true>(p);
+    set_fused_smem_t<8, kMaxN, kMaxBasis, kMaxN, 4, 3, false, true>(p);
     if (tc) {
-      set_fused_smem_t<4, kMaxN, kMaxBasis, kMaxN, 4, 2, true>(p);
-      set_fused_smem_t<8, kMaxN, kMaxBasis, kMaxN, 4, 2, true>(p);
+      set_fused_smem_t<4, kMaxN, kMaxBasis, kMaxN, 4, 2, true, true>(p);
+      set_fused_smem_t<8, kMaxN, kMaxBasis, kMaxN, 4, 2, true, true>(p);
     }
   }
 }
@@ -2305,11 +2330,11 @@ void launch_filter(Engine& e, int N, cudaStream_t s)
   }
 }
 
-// The descriptor kernel evaluates the angular partial forces itself (small
-// shape, Verlet rows, when the autotuner picked it).
+// The descriptor kernel evaluates the angular partial forces itself (degrees
+// <= 4, Verlet rows, when the autotuner picked it).
 bool fused_angular_force(const Engine& e)
 {
-  return e.fuse_f12 && !e.use_xr && small_shape(e.params);
+  return e.fuse_f12 && !e.use_xr && !high_degree(e.params);
 }
 
 void launch_descriptor(Engine& e, int N, const double*, const int*, cudaStream_t stream)
@@ -2322,10 +2347,10 @@ void launch_descriptor(Engine& e, int N, const double*, const int*, cudaStream_t
   else if (e.group == 16 && fused_wide_groups(e)) launch_fused_wide<16>(e, N, stream);
   else if (e.group >= 8) {
     if (small) launch_fused_small<8>(e, N, stream);
-    else launch_fused_g<8, kMaxN, kMaxBasis, kMaxN, 4, 2>(e, N, stream);
+    else launch_fused_general<8>(e, N, stream);
   } else {
     if (small) launch_fused_small<4>(e, N, stream);
-    else launch_fused_g<4, kMaxN, kMaxBasis, kMaxN, 4, 2>(e, N, stream);
+    else launch_fused_general<4>(e, N, stream);
   }
   // a single explicit-row system: the gather evaluates both directed angular
   // forces itself; a batch's structures that are not small take f12 here

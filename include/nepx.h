@@ -319,21 +319,23 @@ int nepx_set_precision(nepx_t* handle, int mode);
 
 /*
  * Launch choices of the force kernels, as NEPX_TUNING_FIELDS ints:
- *   [0] lanes per center of the typewise filter (4 or 8)
- *   [1] lanes per center of the descriptor kernel (4 or 8)
- *   [2] CTAs per SM the descriptor kernel is built for (3 or 4; the
- *       tensor-core build runs at 3 whatever is set)
- *   [3] lanes per center of the angular-force kernel (4 or 8)
- *   [4] lanes per center of the gather (4 or 8)
+ *   [0] lanes per center of the typewise filter (4, 8, 16 or 32)
+ *   [1] lanes per center of the descriptor kernel (4, 8, 16 or 32)
+ *   [2] CTAs per SM the descriptor kernel is built for (3 or 4; models with
+ *       n_max > 4 or basis > 8 run their two builds at 2 and 3, and the
+ *       tensor-core build has one)
+ *   [3] lanes per center of the angular-force kernel (4, 8, 16 or 32)
+ *   [4] lanes per center of the gather (4, 8, 16 or 32)
  *   [5] 1: the descriptor kernel evaluates the angular partial forces itself
- *       (models with n_max <= 4, basis <= 8, l_max <= 4, on the Verlet-row
- *       path), 0: k_angular_f12 does
+ *       (models with l_max <= 4, on the Verlet-row path), 0: k_angular_f12 does
  *   [6] the Verlet-row gather's build (models with l_max <= 4): 3 = unheld
- *       (about 80 registers, three CTAs of 256 per SM), 4 = held to four CTAs
- *       (64 registers, some spills, a third more warps)
- * The first compute of a handle times the variants and keeps the fastest
- * (the autotuner; its picks are shared by the handles of the process and,
- * with NEPX_TUNE_FILE set, kept in that file).  nepx_get_tuning reports the
+ *       (three CTAs of 256 per SM), 4 = held to four CTAs (64 registers, a
+ *       third more warps)
+ * 16 and 32 lanes run as 8 where a kernel has no build of them for the model.
+ * Below 4,096 atoms the first compute of a handle sets them by the size;
+ * otherwise it times the variants and keeps the fastest (the autotuner).  The
+ * picks are shared by the handles of the process and, with NEPX_TUNE_FILE set,
+ * kept in that file.  nepx_get_tuning reports the
  * current choices and *tuned = 1 once they are fixed.  nepx_set_tuning fixes
  * them for every later call on the handle (no timing runs), for example to
  * repeat a run's summation order bit for bit; values outside the lists
