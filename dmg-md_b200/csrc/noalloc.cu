@@ -72,6 +72,20 @@ struct Carver {
   }
 };
 
+// Bytes of alpha, rounded up, and of it and the site energies.
+size_t alpha_bytes(const nepx::Engine& e, size_t N)
+{
+  return (sizeof(float) * N * e.params.T * nepx::alpha_stride(e.params) + 255) & ~size_t(255);
+}
+
+// Alpha and the site energies lie over the Verlet rows where these are large
+// enough: every call builds the rows anew, and the filter has read them before
+// the descriptor kernel writes either.
+bool over_verlet_rows(const nepx::Engine& e, size_t N)
+{
+  return alpha_bytes(e, N) + sizeof(double) * N <= sizeof(int) * N * e.nbr.mn_v;
+}
+
 size_t bytes_needed(const nepx::Engine& e, int n)
 {
   Carver c{nullptr};
@@ -96,9 +110,11 @@ size_t bytes_needed(const nepx::Engine& e, int n)
   c.take<double>(3 * N);        // x0
   c.take<nepx::Site>(N);
   c.take<float>(N * e.params.nR);
-  c.take<float>(N * e.params.T * nepx::alpha_stride(e.params));
   c.take<float4>(N * std::max(nb.mn_a, 2));
-  c.take<double>(N);
+  if (!over_verlet_rows(e, N)) {
+    c.take<unsigned char>(alpha_bytes(e, N));
+    c.take<double>(N);
+  }
   c.take<float>(N * e.params.nA * e.params.nlm);
   return c.used;
 }
@@ -202,10 +218,14 @@ extern "C" int nepx_compute_noalloc(nepx_t* h, const nepx_box* box, int n, const
     nb.cell_cap = static_cast<int>(cells);
     e.scratch.sites = c.take<nepx::Site>(N);
     e.scratch.qrad = c.take<float>(N * e.params.nR);
-    e.scratch.alpha = c.take<float>(N * e.params.T * nepx::alpha_stride(e.params));
     e.scratch.f12 = c.take<float4>(N * std::max(nb.mn_a, 2));
     nb.cell_sites = reinterpret_cast<nepx::Site*>(e.scratch.f12);   // as engine_create has it
-    e.scratch.pe_ann = c.take<double>(N);
+    unsigned char* spent = over_verlet_rows(e, N) ? reinterpret_cast<unsigned char*>(nb.nl_v)
+                                                  : c.take<unsigned char>(alpha_bytes(e, N));
+    e.scratch.alpha = reinterpret_cast<float*>(spent);
+    e.scratch.pe_ann = over_verlet_rows(e, N)
+                         ? reinterpret_cast<double*>(spent + alpha_bytes(e, N))
+                         : c.take<double>(N);
     e.scratch.acoef = c.take<float>(N * e.params.nA * e.params.nlm);
     e.capacity = n;
     e.tuned = true;      // keeps the handle's kernel variants; no timing runs here
