@@ -1,9 +1,11 @@
 // nep_force.cu -- NEP energy, force and virial on sm_100a.
 //
-// Four kernels per force call, each giving a group of G lanes (G = 4 or 8,
-// chosen by the autotuner in engine.cu) to one center; every phase is local
-// to the group, so no CTA-wide barrier follows the set-up (except in the
-// tensor-core ANN, whose MMAs span the CTA's centers).
+// Three kernels per force call (four where k_angular_f12 runs by itself), each
+// giving a group of G lanes to one center: as the autotuner in engine.cu
+// finds (4 or 8, small systems' gather also 32), by a rule on the size below
+// 4096 atoms (up to 32).  Every phase is local to the group, so no CTA-wide barrier
+// follows the set-up (except in the tensor-core ANN, whose MMAs span the
+// CTA's centers).
 //
 //  k_filter_radial  one sweep over the center's sorted Verlet row applies the
 //    reference's FP32 typewise predicate (nep.cu:503-561), writes the radial
@@ -31,9 +33,9 @@
 //    find_partial_force_angular (nep.cu:890-991).
 //  k_gather  radial pair force from both site energies with the per-atom
 //    alpha coefficients (w_ij = sum_k f'_k(d) alpha_i[tj][k]), the angular
-//    exchange F_i += f12(i,j) - f12(j,i) with the reverse slot found by binary
-//    search (reverse_slot) in j's sorted row (explicit rows: both directed forces evaluated
-//    here), ZBL, and the per-atom virial W_i = sum_j r_ij (x) f_ji.
+//    exchange F_i += f12(i,j) - f12(j,i) with the reverse slot found in j's
+//    sorted row through its row of heads (reverse_slot; explicit rows: both
+//    directed forces evaluated here), ZBL, and the per-atom virial W_i = sum_j r_ij (x) f_ji.
 //    Reference: find_force_radial (nep.cu:756-881), gpu_find_force_many_body
 //    (potential.cu:81-210), find_force_ZBL (nep.cu:996-1111).
 //
@@ -2009,13 +2011,14 @@ void launch_fused_t(Engine& e, int N, cudaStream_t s)
   launch_fused_tx<G, NRM, KM, NAM, XR, LMAX, MINB, TC, FF, false>(e, N, s);
 }
 
-// Dynamic shared memory above the default limit (many types): raised for the kernel.
+// Dynamic shared memory above the default limit: the kernel is allowed all an SM
+// has, once and for every handle (a limit of one model's bytes would fall below
+// what another handle's model needs).
 template <typename K>
 void allow_smem(K kernel, size_t bytes)
 {
   if (bytes > 48 * 1024)
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(bytes));
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 
 // The mixed precisions take the FAST builds of the filter, angular-force and
@@ -2096,18 +2099,20 @@ void set_fused_smem_t(const ModelParams& p)
 {
   const int bytes =
     fused_layout(p, kBlock / G, (KM + 3) & ~3, fused_smem_budget(MINB), TC).total_bytes;
-  auto limit = [](auto kernel, int n) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
-  };
-  limit(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, false, false>, bytes);
-  limit(k_nep_fused<G, NRM, KM, NAM, true, LMAX, MINB, TC, false, false>, bytes);
-  if constexpr (FFI)
-    limit(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, true, false>, bytes);
+  // (only the builds this model runs, and only above the default limit: the
+  // calls add up in the making of a handle)
   if constexpr (KM == kSmallK && LMAX == 4) {
-    limit(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, false, true>, bytes);
-    limit(k_nep_fused<G, NRM, KM, NAM, true, LMAX, MINB, TC, false, true>, bytes);
-    limit(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, true, true>, bytes);
+    if (exact_shape(p)) {
+      allow_smem(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, false, true>, bytes);
+      allow_smem(k_nep_fused<G, NRM, KM, NAM, true, LMAX, MINB, TC, false, true>, bytes);
+      allow_smem(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, true, true>, bytes);
+      return;
+    }
   }
+  allow_smem(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, false, false>, bytes);
+  allow_smem(k_nep_fused<G, NRM, KM, NAM, true, LMAX, MINB, TC, false, false>, bytes);
+  if constexpr (FFI)
+    allow_smem(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, true, false>, bytes);
 }
 
 template <int G>
@@ -2116,12 +2121,10 @@ void set_fused_smem_wide(const ModelParams& p)
   constexpr int n = kSmallN, k = kSmallK;
   const int bytes =
     fused_layout(p, kBlock / G, (k + 3) & ~3, fused_smem_budget(3), false).total_bytes;
-  auto limit = [&](auto kernel) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  };
-  limit(k_nep_fused<G, n, k, n, true, 4, 3, false, false, true>);
-  limit(k_nep_fused<G, n, k, n, false, 4, 3, false, true, true>);
-  limit(k_nep_fused<G, n, k, n, false, 4, 3, false, false, true>);
+  if (!exact_shape(p)) return;
+  allow_smem(k_nep_fused<G, n, k, n, true, 4, 3, false, false, true>, bytes);
+  allow_smem(k_nep_fused<G, n, k, n, false, 4, 3, false, true, true>, bytes);
+  allow_smem(k_nep_fused<G, n, k, n, false, 4, 3, false, false, true>, bytes);
 }
 
 template <int G, int KM, int NAM, int ROWS, int LMAX, int GMINB, bool FAST>

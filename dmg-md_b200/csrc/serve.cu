@@ -183,7 +183,7 @@ __global__ void k_vv1_batch(int T, const int* __restrict__ sid, const int* __res
   }
 }
 
-// Second half kick (md.cu k_vv2_thermo without the thermo sums).
+// Second half kick (md.cu k_vv2_ensemble without the sums and the ensemble).
 __global__ void k_vv2_batch(int T, const int* __restrict__ sid, const int* __restrict__ sflag,
                             const double* __restrict__ sdt, const double* __restrict__ mass,
                             const double* __restrict__ force, double* vel)
