@@ -978,9 +978,10 @@ def main():
     dev_ms, st, clock_info, nchunks = timed_md(pot, sysd, args, rank, ranks, flush, clocks)
     value, dev_ms = replica_rate(n, K, dev_ms, ranks)
     # k_vv1 (with the skin check), k_neighbor_rebuild (returns at once unless
-    # a rebuild is due), the force kernels, k_vv2_thermo, k_ensemble, k_scale;
-    # NHC adds two
-    kernels_per_step = 5 + len(force_kernels(pot)) + (2 if kind == "nvt_nhc" else 0)
+    # a rebuild is due), the force kernels, k_vv2_ensemble; k_scale except in
+    # NVE; NHC adds two
+    kernels_per_step = 3 + len(force_kernels(pot)) + (0 if kind == "nve" else 1)
+    kernels_per_step += 2 if kind == "nvt_nhc" else 0
     # per call (chunk): k_mark_call before the step graphs and k_publish after
     # them; the L2-flush fills are torch's, not counted
     launches = K * kernels_per_step + 2 * nchunks
