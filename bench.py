@@ -81,9 +81,9 @@ K_B = 8.617343e-5
 # per SM: the builds the autotuner picks for this model), dram__bytes_read.sum
 # + dram__bytes_write.sum of one ncu-captured launch each on the large-carbon
 # system at 1,000,000 atoms (--ncell 50), divided by its atoms (traffic grows
-# with the atoms processed).  An earlier build's capture; the present kernels
-# moved 4.2 kB per atom on 208,568 atoms.  Keyed by workload and the kernel list; another
-# form reports no traffic.
+# with the atoms processed).  An earlier build's capture: the present kernels
+# move 4.66 kB per atom (the filter also writes the angular edges).  Keyed by
+# workload and the kernel list; another form reports no traffic.
 TRAFFIC_PER_ATOM = {
     ("carbon8m", ("k_filter_radial", "k_nep_fused", "k_gather")):
         (701.6 + 412.2 + 349.1 + 567.1 + 1359.3 + 292.3) * 1e6 / 1.0e6}
