@@ -314,15 +314,20 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b)
 
 // Cutoff function fc = (1 + cos(pi d / rc)) / 2 and its d-derivative.
 // On the one period's half that occurs, x = d / rc in [0, 1), both are short
-// polynomials without a range reduction:
-//   fc  = 1/2 - y P(y^2), y = x - 1/2, since cos(pi x) = -sin(pi y);
-//   fc' = t R(t) / rc, t = x (1 - x), since sin(pi x) is an entire function of
-//         t that vanishes with it (so it keeps its relative accuracy at rc).
-// P and R are least-maximum-error fits by iterated weighted least squares on
+// polynomials in t = x (1 - x) without a range reduction:
+//   fc  = (1 - x) - y t S(t), y = x - 1/2: the cosine less its chord, which vanishes
+//         with t. w = 1 - x is rounded below 1/2, and what it loses joins the
+//         small term, so the sum is rounded once.
+//   fc' = t R(t) / rc, since sin(pi x) is an entire function of t that vanishes with
+//         it (so it keeps its relative accuracy at rc). R's constant -pi^2/2 is taken
+//         in two parts, its leading product inside the last fma.
+// S and R are least-maximum-error fits by iterated weighted least squares on
 // Chebyshev nodes with the leading coefficients rounded first (residual 3e-9 and
-// 1e-9).  Against 64 bits over [0, 1): fc 1.8e-8 rms (cospi in 32 bits: 1.6e-8),
-// fc' 4.8e-8 relative rms (sinpi: 5.9e-8); about 15 instructions for the pair
-// where sincospif took some 30.
+// 1e-9).  Against 64 bits, over every float of [2^-10, 1) (in brackets the same
+// from sincospif, which took some 30 instructions for the pair; these take about
+// 18): fc at most 5.5e-8 (5.6e-8), rms 1.7e-8 (2.2e-8); fc' at most 1.2e-7 (1.7e-7)
+// relative, rms 3.6e-8 (4.9e-8).  An earlier fit, fc = 1/2 - y P(y^2) without the
+// chord, reached 8.1e-8 and 1.8e-7.
 // FAST (the mixed-precision kernels): sine and cosine from the hardware
 // approximations (absolute error about 4e-7 on [0, pi)).
 template <bool FAST = false>
@@ -336,20 +341,18 @@ __device__ __forceinline__ void cutoff_fc(float rc, float rcinv, float d, float&
       fcp = -1.5707963f * s * rcinv;
     } else {
       const float x = d * rcinv;
-      const float y = x - 0.5f, y2 = y * y;
-      float p = 0.03901020435f;
-      p = fmaf(p, y2, -0.2992585005f);
-      p = fmaf(p, y2, 1.27506292f);
-      p = fmaf(p, y2, -2.58385706f);
-      p = fmaf(p, y2, 1.57079637f);
-      fc = fmaf(-y, p, 0.5f);
       const float t = fmaf(-x, x, x);
-      float r = -0.032579802f;
-      r = fmaf(r, t, -0.324012071f);
-      r = fmaf(r, t, -1.75180531f);
-      r = fmaf(r, t, -4.93482113f);
-      r = fmaf(r, t, -4.93480206f);
-      fcp = t * r * rcinv;
+      float p = 0.0383364521f;
+      p = fmaf(p, t, 0.260538638f);
+      p = fmaf(p, t, 1.06520951f);
+      p = fmaf(p, t, 2.0f);
+      const float w = 1.0f - x;
+      fc = w + fmaf((0.5f - x) * t, p, (1.0f - w) - x);
+      float r = -0.0378732346f;
+      r = fmaf(r, t, -0.321397096f);
+      r = fmaf(r, t, -1.75220692f);
+      r = fmaf(r, t, -4.93480158f);
+      fcp = fmaf(t, -4.93480206f, t * fmaf(r, t, -1.45185794e-7f)) * rcinv;
     }
   } else {
     fc = 0.0f;
@@ -357,11 +360,12 @@ __device__ __forceinline__ void cutoff_fc(float rc, float rcinv, float d, float&
   }
 }
 
-// Edge length d and 1 / d from d^2.  One hardware reciprocal square root y (2
-// ulp), then one correction each of d2 y and y by their exact residuals (fma):
-// d comes out as the correctly rounded root in all but a few of a thousand
-// arguments and 1 / d within 1 ulp, in 7 instructions without the slow-path
-// branches that the root and the division bring.  FAST takes y itself.
+// Edge length d and 1 / d from d^2: from one hardware reciprocal root y (2 ulp)
+// by Markstein's method (P. W. Markstein, IBM J. Res. Dev. 34 (1990) 111), a Newton
+// step of the root from d2 y and one of the reciprocal from y, each on a residual that
+// an fma gives exactly.  7 instructions without a branch.  Over every float of two
+// neighbouring binades d is sqrtf's and 1 / d within the error of the division
+// (8.9e-8 against 64 bits, both).  FAST takes y itself.
 template <bool FAST>
 __device__ __forceinline__ void edge_length(float d2, float& d, float& dinv)
 {

@@ -310,8 +310,8 @@ int nepx_md_device_state(nepx_md_t* md, double** d_pos, double** d_vel, double**
  * and force kernels (models with n_max <= 4, basis <= 8, l_max <= 4) take
  * the hardware approximations of 1/sqrt (edge lengths), 1/x and sine/cosine
  * (the cutoff function), 2 ulp or about 4e-7 absolute, in place of the
- * correctly rounded functions the FP32 mode keeps for parity with the
- * reference.  NEPX_ERR_UNSUPPORTED for models with dim >
+ * FP32 mode's functions, whose errors are no larger than those of the sqrtf,
+ * division and sincospif that the reference calls.  NEPX_ERR_UNSUPPORTED for models with dim >
  * 128 or more than 256 hidden units.  No counterpart in the reference (its
  * ANN is FP32 only).
  */
