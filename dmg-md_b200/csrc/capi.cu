@@ -181,7 +181,7 @@ int nepx_compute(nepx_t* h, const nepx_box* box, int n, const int* d_type, const
   e.staged_box = &b;   // the neighbour update's launch takes the box along
   nepx::launch_neighbor_update(e, n, d_pos, d_type, rebuild, s);
   e.staged_box = nullptr;
-  if (!e.tuned) nepx::engine_autotune(e, n, d_pos, d_type, s);
+  nepx::engine_choose(e, n, d_pos, d_type, s, nepx::ChoiceScope::kByCall);
   nepx::launch_force(e, n, d_pos, d_type, d_pe, d_force, d_virial,
                      (flags & NEPX_ACCUMULATE) != 0, s);
   if (cudaPeekAtLastError() != cudaSuccess) return cuda_fail(h, "kernel launch");
@@ -316,7 +316,7 @@ int nepx_set_tuning(nepx_t* h, const int* v)
   e.gather_group = v[4];
   e.fuse_f12 = v[5] == 1;
   e.gather_minb = v[6];
-  e.tuned = true;
+  e.tuned = e.pinned = true;
   return NEPX_OK;
 }
 

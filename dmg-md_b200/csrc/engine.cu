@@ -235,21 +235,22 @@ struct TuneKey {
   int v[14];
   bool operator==(const TuneKey& o) const { return std::memcmp(v, o.v, sizeof(v)) == 0; }
 };
-struct TuneVal {
-  int filter_group, group, fused_minb, f12_group, gather_group, fuse_f12, gather_minb;
-};
-
 std::mutex g_tune_mu;
-std::vector<std::pair<TuneKey, TuneVal>> g_tune;
+std::vector<std::pair<TuneKey, LaunchChoices>> g_tune;
 bool g_tune_loaded = false;
+
+int size_class(int N)
+{
+  int c = 0;
+  while (c < 30 && (1 << (c + 1)) <= N) ++c;   // floor(log2 N)
+  return c;
+}
 
 TuneKey tune_key(const Engine& e, int N)
 {
   const ModelParams& p = e.params;
-  int size_class = 0;
-  while ((1 << (size_class + 1)) <= N) ++size_class;   // floor(log2 N)
   TuneKey k{{e.device, e.use_xr ? 1 : 0, e.precision, p.T, p.nR, p.nA, p.kR, p.kA, p.L_max,
-             p.dim, p.H, p.num_inv, size_class, 3}};
+             p.dim, p.H, p.num_inv, size_class(N), 3}};
   return k;
 }
 
@@ -264,23 +265,25 @@ void tune_load_file()
   while (std::getline(in, line)) {
     std::istringstream ls(line);
     TuneKey k;
-    TuneVal v;
+    LaunchChoices v;
+    int fuse = 0;
     bool ok = true;
     for (int& x : k.v) ok = ok && static_cast<bool>(ls >> x);
     ok = ok && static_cast<bool>(ls >> v.filter_group >> v.group >> v.fused_minb >> v.f12_group >>
-                                 v.gather_group >> v.fuse_f12 >> v.gather_minb);
+                                 v.gather_group >> fuse >> v.gather_minb);
+    v.fuse_f12 = fuse != 0;
     // only the shapes the launchers instantiate; anything else is ignored
     ok = ok && lanes_built(v.filter_group) && lanes_built(v.group) && lanes_built(v.f12_group) &&
          lanes_built(v.gather_group) && (v.fused_minb == 3 || v.fused_minb == 4) &&
-         (v.fuse_f12 == 0 || v.fuse_f12 == 1) && (v.gather_minb == 3 || v.gather_minb == 4);
+         (fuse == 0 || fuse == 1) && (v.gather_minb == 3 || v.gather_minb == 4);
     if (ok) g_tune.emplace_back(k, v);
   }
 }
 
-bool tune_lookup(const TuneKey& k, TuneVal& v)
+bool tune_lookup(const TuneKey& k, LaunchChoices& v, bool load_file)
 {
   std::lock_guard<std::mutex> lock(g_tune_mu);
-  tune_load_file();
+  if (load_file) tune_load_file();
   for (const auto& kv : g_tune)
     if (kv.first == k) {
       v = kv.second;
@@ -289,7 +292,7 @@ bool tune_lookup(const TuneKey& k, TuneVal& v)
   return false;
 }
 
-void tune_store(const TuneKey& k, const TuneVal& v)
+void tune_store(const TuneKey& k, const LaunchChoices& v)
 {
   std::lock_guard<std::mutex> lock(g_tune_mu);
   for (const auto& kv : g_tune)
@@ -299,54 +302,64 @@ void tune_store(const TuneKey& k, const TuneVal& v)
     std::ofstream out(path, std::ios::app);
     for (int x : k.v) out << x << ' ';
     out << v.filter_group << ' ' << v.group << ' ' << v.fused_minb << ' ' << v.f12_group << ' '
-        << v.gather_group << ' ' << v.fuse_f12 << ' ' << v.gather_minb << '\n';
+        << v.gather_group << ' ' << (v.fuse_f12 ? 1 : 0) << ' ' << v.gather_minb << '\n';
   }
 }
 
-}  // namespace
+LaunchChoices& choices(Engine& e) { return e; }
 
-void engine_autotune(Engine& e, int N, const double* pos, const int* type, cudaStream_t stream)
+// A small system (below kWideAtoms): lanes by size, nothing timed.  A kernel's time
+// is then the chain of one center's edges plus what each center costs the chip, and
+// the best group narrows as the atoms fill it (us, lanes 4 8 16 32, the other
+// kernel at 8):
+//   descriptor kernel   water 210: 32 21 17 14;  carbon 1,000: 32 28 26 28;
+//                       4,096: 36 34 40 51;  8,000: 44 48 56 77
+//   filter              water 600: 45 34 28 26;  1,551: 50 38 32 32;
+//                       carbon 4,096: 36 34 34 38;  8,000: 50 48 54 63
+//   gather              water 1,551: 44 30 23 14;  carbon 4,096: 34 24 21 19;
+//                       8,000: 35 25 29 26
+// (1,551 water atoms in the descriptor kernel: 44 38 38 36.)  A rule also gives
+// every process of a small system the same sums; its lines are powers of two
+// because the picks are kept by size class.
+LaunchChoices small_choices(Engine& e, int N)
 {
-  const TuneKey key = tune_key(e, N);
-  TuneVal known{};
-  if (tune_lookup(key, known)) {
-    e.filter_group = known.filter_group;
-    e.group = known.group;
-    e.fused_minb = known.fused_minb;
-    e.f12_group = known.f12_group;
-    e.gather_group = known.gather_group;
-    e.fuse_f12 = known.fuse_f12 != 0;
-    e.gather_minb = known.gather_minb;
-    e.tuned = true;
-    return;
-  }
-  if (N < kWideAtoms) {
-    // a small system: lanes by size, nothing timed.  A kernel's time is then the
-    // chain of one center's edges plus what each center costs the chip, and the
-    // best group narrows as the atoms fill it (us, lanes 4 8 16 32, the other
-    // kernel at 8):
-    //   descriptor kernel   water 210: 32 21 17 14;  carbon 1,000: 32 28 26 28;
-    //                       4,096: 36 34 40 51;  8,000: 44 48 56 77
-    //   filter              water 600: 45 34 28 26;  1,551: 50 38 32 32;
-    //                       carbon 4,096: 36 34 34 38;  8,000: 50 48 54 63
-    //   gather              water 1,551: 44 30 23 14;  carbon 4,096: 34 24 21 19;
-    //                       8,000: 35 25 29 26
-    // (1,551 water atoms in the descriptor kernel: 44 38 38 36.)  A rule also
-    // gives every process of a small system the same sums; its lines are powers of
-    // two because the picks are kept by size class.
-    e.filter_group = N < 1024 ? 32 : 16;
-    e.group = !fused_wide_groups(e) ? 8 : N < 512 ? 32 : N < 1024 ? 16 : 8;
-    e.fused_minb = 3;
-    e.f12_group = 8;
-    e.gather_group = 32;
-    e.gather_minb = 3;
-    e.fuse_f12 = true;
-    e.fuse_f12 = fused_angular_force(e);
-    e.tuned = true;
-    tune_store(key, TuneVal{e.filter_group, e.group, e.fused_minb, e.f12_group, e.gather_group,
-                            e.fuse_f12 ? 1 : 0, e.gather_minb});
-    return;
-  }
+  LaunchChoices c;
+  c.filter_group = N < 1024 ? 32 : 16;
+  c.group = !fused_wide_groups(e) ? 8 : N < 512 ? 32 : N < 1024 ? 16 : 8;
+  c.fused_minb = 3;
+  c.f12_group = 8;
+  c.gather_group = 32;
+  c.gather_minb = 3;
+  const bool was = e.fuse_f12;
+  e.fuse_f12 = true;
+  c.fuse_f12 = fused_angular_force(e);
+  e.fuse_f12 = was;
+  return c;
+}
+
+// A batch handle or server for many atoms whose first step holds few: nothing to
+// time on yet, and a small step's lanes would stay for the full ones.  Lanes that
+// serve both (ms; 48 requests, some 13,000 atoms a step, and one batch of 248,000
+// atoms; the gather at 4 8 16 32 lanes, then the descriptor kernel):
+//   descriptor kernel at 4:  29.9 25.9 24.7 24.0;  2.67 2.68 2.74 2.90
+//   gather at 16:            24.7 25.4 25.4 25.4;  2.74 2.86 3.34 4.08
+// (the gather of a small box evaluates both angular forces of an edge, so it gains
+// from more lanes for longer than the descriptor kernel).
+LaunchChoices filling_choices(const Engine& e)
+{
+  LaunchChoices c;
+  c.group = 4;
+  c.fused_minb = fused_wide_groups(e) ? 4 : 3;
+  c.f12_group = 8;
+  c.gather_group = 16;
+  return c;
+}
+
+// The launch variants timed on the given system, the fastest left in e; the
+// 32-lane gather only for wide_gather.
+void time_variants(Engine& e, int N, const double* pos, const int* type, cudaStream_t stream,
+                   bool wide_gather)
+{
   const int groups[2] = {4, 8};   // candidate lanes per center
   cudaEvent_t a, b;
   cudaEventCreate(&a);
@@ -416,8 +429,8 @@ void engine_autotune(Engine& e, int N, const double* pos, const int* type, cudaS
   float best_g = 1e30f;
   int pick_g = 8, pick_gm = 3;
   const int gm_last = !e.use_xr && e.params.L_max <= 4 ? 4 : 3;
-  const int gather_lanes[3] = {4, 8, 32};   // 8,000 carbon atoms: 35 25 23 us
-  const int n_lanes = N < 16384 ? 3 : 2;
+  const int gather_lanes[3] = {4, 8, 32};
+  const int n_lanes = wide_gather ? 3 : 2;
   for (int gm = 3; gm <= gm_last; ++gm)
     for (int k = 0; k < n_lanes; ++k) {
       e.gather_minb = gm;
@@ -444,9 +457,6 @@ void engine_autotune(Engine& e, int N, const double* pos, const int* type, cudaS
   e.f12_group = pick_a;
   e.gather_group = pick_g;
   e.fuse_f12 = pick_ff;
-  e.tuned = true;
-  tune_store(key, TuneVal{e.filter_group, e.group, e.fused_minb, e.f12_group, e.gather_group,
-                          e.fuse_f12 ? 1 : 0, e.gather_minb});
   if (std::getenv("NEPX_VERBOSE"))
     std::fprintf(stderr,
                  "nepx autotune (N=%d): filter G=%d, fused G=%d at %d CTAs/SM, angular force "
@@ -454,6 +464,59 @@ void engine_autotune(Engine& e, int N, const double* pos, const int* type, cudaS
                  N, e.filter_group, e.group, e.fused_minb,
                  e.fuse_f12 ? "in the descriptor kernel" : "own kernel", e.f12_group,
                  e.gather_group, e.gather_minb);
+}
+
+bool can_time(cudaStream_t stream)
+{
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) == cudaSuccess)
+    return status == cudaStreamCaptureStatusNone;
+  cudaGetLastError();   // the legacy stream while another stream is capturing
+  return false;
+}
+
+}  // namespace
+
+void engine_choose(Engine& e, int N, const double* pos, const int* type, cudaStream_t stream,
+                   ChoiceScope scope, bool may_time)
+{
+  if (e.pinned) return;
+  const bool by_handle = scope == ChoiceScope::kByHandle;
+  // the size that sets the choice: the call's, or the largest the handle serves
+  const int n = by_handle ? e.capacity : N;
+  const Engine::ChosenFor want{scope, by_handle ? -1 : size_class(n), e.use_xr};
+  if (e.tuned && e.chosen_for == want) return;
+  const int band = n < kWideAtoms ? 0 : n < kGatherWideAtoms ? 1 : 2, path = e.use_xr ? 1 : 0;
+  const TuneKey key = tune_key(e, n);
+  LaunchChoices known;
+  bool fixed = true;
+  if (by_handle && e.has_by_handle) {
+    choices(e) = e.by_handle;
+  } else if (tune_lookup(key, known, may_time)) {
+    choices(e) = known;
+  } else if (band == 0) {
+    choices(e) = small_choices(e, n);
+    if (may_time) tune_store(key, choices(e));
+  } else if (by_handle && N < kWideAtoms) {
+    choices(e) = filling_choices(e);
+  } else if (!by_handle && e.has_timed[path][band]) {
+    choices(e) = e.timed[path][band];
+  } else if (may_time && can_time(stream)) {
+    time_variants(e, N, pos, type, stream, band == 1);
+    e.timed[path][band] = e;
+    e.has_timed[path][band] = true;
+    tune_store(key, choices(e));
+  } else {
+    const int other = band == 1 ? 2 : 1;
+    choices(e) = e.has_timed[path][other] ? e.timed[path][other] : LaunchChoices{};
+    fixed = false;
+  }
+  e.tuned = fixed;
+  e.chosen_for = want;
+  if (by_handle && fixed) {
+    e.by_handle = e;
+    e.has_by_handle = true;
+  }
 }
 
 namespace {
@@ -530,7 +593,10 @@ std::string engine_set_precision(Engine& e, int mode)
     set_fused_smem_limits(p);
     if (cudaGetLastError() != cudaSuccess) return "CUDA error setting up the tensor-core ANN";
   }
-  if (e.precision != mode) e.tuned = false;
+  if (e.precision != mode) {
+    e.tuned = e.pinned = e.has_by_handle = false;
+    std::memset(e.has_timed, 0, sizeof(e.has_timed));
+  }
   e.precision = mode;
   return "";
 }

@@ -97,7 +97,24 @@ struct ExplicitRows {
   BatchVerlet bv;
 };
 
-struct Engine {
+// How the force kernels are launched (nepx_get_tuning).
+struct LaunchChoices {
+  int group = 4;             // lanes per center in the fused kernel
+  int fused_minb = 3;        // CTAs per SM the fused kernel is built for
+  int filter_group = 8;      // lanes per center in the typewise filter
+  int f12_group = 4;         // lanes per center in the angular-force kernel
+  int gather_group = 8;      // lanes per center in the gather
+  int gather_minb = 3;       // Verlet-row gather build: 3 unheld, 4 held to four CTAs
+  bool fuse_f12 = false;     // the descriptor kernel evaluates f12 itself
+};
+
+// Whose launch choices a call takes (engine_choose).  kByCall: those of its own
+// size.  kByHandle: one set for the handle's life, by its capacity -- the sums of
+// a structure in a batch or a server must not depend on what shares its launch,
+// and the explicit-row trajectories of an md and of a server are the same.
+enum class ChoiceScope { kByCall, kByHandle };
+
+struct Engine : LaunchChoices {
   NepModel model;
   ModelParams params{};
   int capacity = 0;          // atoms the buffers are sized for
@@ -124,14 +141,21 @@ struct Engine {
   // launch writes it to the device copy (in place of a launch of its own)
   const Box* staged_box = nullptr;
   int last_n = -1;
-  int group = 4;             // lanes per center in the fused kernel (autotuned)
-  int fused_minb = 3;        // CTAs per SM the small-shape fused kernel is built for (autotuned)
-  int filter_group = 8;      // lanes per center in the typewise filter (autotuned)
-  int f12_group = 4;         // lanes per center in the angular-force kernel (autotuned)
-  int gather_group = 8;      // lanes per center in the gather (autotuned)
-  int gather_minb = 3;       // Verlet-row gather build: 3 unheld, 4 held to four CTAs (autotuned)
-  bool fuse_f12 = false;     // the descriptor kernel evaluates f12 itself (autotuned)
-  bool tuned = false;
+  bool tuned = false;        // the launch choices are set for what chosen_for names
+  bool pinned = false;       // ... by nepx_set_tuning, for every later call
+  struct ChosenFor {
+    ChoiceScope scope = ChoiceScope::kByCall;
+    int size_class = -1;     // log2 of the atoms (kByCall)
+    bool xr = false;
+    bool operator==(const ChosenFor& o) const
+    {
+      return scope == o.scope && size_class == o.size_class && xr == o.xr;
+    }
+  } chosen_for;
+  // what this handle has timed, per row path and size band (engine_choose), and
+  // its one set for batches
+  LaunchChoices timed[2][3], by_handle;
+  bool has_timed[2][3] = {}, has_by_handle = false;
   std::string error;
 };
 
@@ -147,8 +171,11 @@ size_t fused_tc_smem_bytes(const ModelParams& p);
 // a kernel has no build for the model.
 inline bool lanes_built(int g) { return g == 4 || g == 8 || g == 16 || g == 32; }
 // Systems below this many atoms take their lanes from a rule on the size
-// (engine_autotune); from there on the chip is full at 4 or 8 lanes.
+// (engine_choose); from there on the chip is full at 4 or 8 lanes.
 constexpr int kWideAtoms = 4096;
+// Below this many the gather's 32-lane groups are timed too (8,000 carbon atoms,
+// lanes 4 8 32: 35 25 23 us).
+constexpr int kGatherWideAtoms = 16384;
 // True when the descriptor kernel has 16- and 32-lane groups for this model
 // and precision.
 bool fused_wide_groups(const Engine& e);
@@ -156,20 +183,27 @@ bool fused_wide_groups(const Engine& e);
 // per SM, Engine::fused_minb) for this model's shape.
 bool fused_occupancy_variants(const ModelParams& p);
 // True when the descriptor kernel writes the angular partial forces itself
-// (Engine::fuse_f12 on a small-shape model and Verlet rows): no k_angular_f12.
+// (Engine::fuse_f12, degrees <= 4, on Verlet rows): no k_angular_f12.
 bool fused_angular_force(const Engine& e);
+// True when the filter and the gather have 16- and 32-lane groups for this model.
+bool wide_groups(const ModelParams& p);
 void set_fused_smem_limits(const ModelParams& p);
 
-// Takes the lanes of a small system (below kWideAtoms) from its size; otherwise
-// times each kernel variant on the given system (a few calls each, stream
-// synchronised) and keeps the fastest: the lane-group size of the filter,
-// descriptor, angular-force and gather kernels, the CTAs per SM of the
-// descriptor kernel and of the gather, and whether the descriptor kernel
-// evaluates the angular partial forces itself.  The picks are kept per (device, model shape, precision, row
-// path, size class log2 N) for every later handle of the process, and in the
-// file NEPX_TUNE_FILE names, when set, across runs.  Neighbour rows must be
-// current.
-void engine_autotune(Engine& e, int N, const double* pos, const int* type, cudaStream_t stream);
+// Sets the launch choices of a call of N atoms: nothing to do while they are those
+// of its size class and row path, or pinned.  A small system (below kWideAtoms)
+// takes its lanes from its size; otherwise each kernel variant is timed on the
+// given system (a few calls each, stream synchronised) and the fastest kept: the
+// lane-group size of the filter, descriptor, angular-force and gather kernels,
+// the CTAs per SM of the descriptor kernel and of the gather, and whether the
+// descriptor kernel evaluates the angular partial forces itself.  A handle times
+// once per row path and size band (below kWideAtoms, below kGatherWideAtoms,
+// above); the picks are kept per (device, model shape, precision, row path, size
+// class log2 N) for every later handle of the process, and in the file
+// NEPX_TUNE_FILE names, when set, across runs.  Neighbour rows must be current.
+// may_time false, or a stream under capture: nothing is timed; what is known, or
+// a default, serves this call (may_time false also allocates no host memory).
+void engine_choose(Engine& e, int N, const double* pos, const int* type, cudaStream_t stream,
+                   ChoiceScope scope, bool may_time = true);
 
 // Loads the potential, uploads it and sizes every buffer for max_atoms.
 std::string engine_create(Engine& e, const std::string& nep_path, int max_atoms);

@@ -902,11 +902,16 @@ int md_enqueue_run(nepx_md* m, int steps, double dt_fs, int thermo_every, double
     if (first_step == 0) nepx::md_init_scalars(md, p, c.T0, tau);
     else nepx::md_continue_scalars(md);
   }
+  const nepx::ChoiceScope scope =
+    md.xr ? nepx::ChoiceScope::kByHandle : nepx::ChoiceScope::kByCall;
   if (!md.forces_valid) {
     nepx::launch_neighbor_update(e, N, md.d_pos, md.d_type, true, s);
-    if (!e.tuned) nepx::engine_autotune(e, N, md.d_pos, md.d_type, s);
+    nepx::engine_choose(e, N, md.d_pos, md.d_type, s, scope);
     nepx::launch_force(e, N, md.d_pos, md.d_type, md.d_pe, md.d_force, md.d_virial, false, s);
     md.forces_valid = true;
+  } else {
+    // the handle may have served a call of another size since the last run
+    nepx::engine_choose(e, N, md.d_pos, md.d_type, s, scope, false);
   }
   e.force_rebuild = true;     // a later nepx_compute on this handle rebuilds
   e.have_box = false;
@@ -1118,7 +1123,8 @@ int nepx_md_compute_forces(nepx_md_t* m)
     rebuild = true;
   }
   nepx::launch_neighbor_update(e, N, md.d_pos, md.d_type, rebuild, s);
-  if (!e.tuned) nepx::engine_autotune(e, N, md.d_pos, md.d_type, s);
+  nepx::engine_choose(e, N, md.d_pos, md.d_type, s,
+                      md.xr ? nepx::ChoiceScope::kByHandle : nepx::ChoiceScope::kByCall);
   nepx::launch_force(e, N, md.d_pos, md.d_type, md.d_pe, md.d_force, md.d_virial, false, s);
   md.forces_valid = true;
   e.force_rebuild = true;     // a later nepx_compute on this handle rebuilds

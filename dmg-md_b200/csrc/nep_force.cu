@@ -2263,6 +2263,8 @@ int alpha_stride(const ModelParams& p)
 
 bool fused_occupancy_variants(const ModelParams& p) { return !high_degree(p); }
 
+bool wide_groups(const ModelParams& p) { return small_shape(p); }
+
 bool fused_wide_groups(const Engine& e) { return exact_shape(e.params) && e.precision == 0; }
 
 // Largest dynamic shared memory a descriptor-kernel variant this model runs needs.

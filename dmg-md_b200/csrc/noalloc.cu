@@ -130,12 +130,14 @@ struct BorrowedBuffers {
   nepx::NeighborState* d_nstate;
   nepx::NeighborBuffers nbr;
   nepx::ForceScratch scratch;
+  nepx::LaunchChoices choices;
+  nepx::Engine::ChosenFor chosen_for;
   int capacity;
   bool tuned, use_xr;
   int precision;
   explicit BorrowedBuffers(nepx::Engine& eng)
     : e(eng), d_box(eng.d_box), d_nstate(eng.d_nstate), nbr(eng.nbr), scratch(eng.scratch),
-      capacity(eng.capacity), tuned(eng.tuned), use_xr(eng.use_xr), precision(eng.precision)
+      choices(eng), chosen_for(eng.chosen_for), capacity(eng.capacity), tuned(eng.tuned), use_xr(eng.use_xr), precision(eng.precision)
   {
   }
   ~BorrowedBuffers()
@@ -144,6 +146,8 @@ struct BorrowedBuffers {
     e.d_nstate = d_nstate;
     e.nbr = nbr;
     e.scratch = scratch;
+    static_cast<nepx::LaunchChoices&>(e) = choices;
+    e.chosen_for = chosen_for;
     e.capacity = capacity;
     e.tuned = tuned;
     e.use_xr = use_xr;
@@ -228,9 +232,10 @@ extern "C" int nepx_compute_noalloc(nepx_t* h, const nepx_box* box, int n, const
                          : c.take<double>(N);
     e.scratch.acoef = c.take<float>(N * e.params.nA * e.params.nlm);
     e.capacity = n;
-    e.tuned = true;      // keeps the handle's kernel variants; no timing runs here
     e.precision = 0;     // FP32 ANN: the mixed path's buffers are not in the static array
     e.use_xr = false;
+    e.tuned = false;     // the choices for this size, without timing runs
+    nepx::engine_choose(e, n, d_pos, d_type, s, nepx::ChoiceScope::kByCall, false);
     // the array keeps the previous call's contents: clear the flags, rebuild
     cudaMemsetAsync(e.d_nstate, 0, sizeof(nepx::NeighborState), s);
     cudaMemsetAsync(nb.gsync, 0, 2 * sizeof(unsigned), s);

@@ -278,7 +278,7 @@ void launch_batch_force(Engine& e, int T, const double* pos, const int* type, do
   e.use_xr = true;
   e.xr.from_box = false;
   launch_explicit_rows(e, T, pos, type, s);
-  if (!e.tuned) engine_autotune(e, T, pos, type, s);
+  engine_choose(e, T, pos, type, s, ChoiceScope::kByHandle);
   launch_force(e, T, pos, type, pe, force, virial, accumulate, s);
   // the Verlet-path state of the handle no longer matches its last box
   e.force_rebuild = true;

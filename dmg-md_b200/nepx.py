@@ -239,7 +239,7 @@ class Potential:
 
     def tuning(self):
         """The force kernels' launch choices (dict of TUNING_FIELDS) and whether
-        they are fixed yet (the autotuner runs at the first compute)."""
+        they are kept (the latest call's; they follow its size)."""
         v = (ctypes.c_int * len(TUNING_FIELDS))()
         tuned = ctypes.c_int(0)
         self._check(lib().nepx_get_tuning(self._h, v, ctypes.byref(tuned)))

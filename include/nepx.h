@@ -332,11 +332,14 @@ int nepx_set_precision(nepx_t* handle, int mode);
  *       (three CTAs of 256 per SM), 4 = held to four CTAs (64 registers, a
  *       third more warps)
  * 16 and 32 lanes run as 8 where a kernel has no build of them for the model.
- * Below 4,096 atoms the first compute of a handle sets them by the size;
- * otherwise it times the variants and keeps the fastest (the autotuner).  The
- * picks are shared by the handles of the process and, with NEPX_TUNE_FILE set,
- * kept in that file.  nepx_get_tuning reports the
- * current choices and *tuned = 1 once they are fixed.  nepx_set_tuning fixes
+ * They follow the size of each call: below 4,096 atoms they are set by it, from
+ * there on a handle's first call of a size times the variants and keeps the
+ * fastest (the autotuner; once per row path below and above 16,384 atoms; not
+ * under stream capture).  Batches, servers and an md on explicit rows keep one set
+ * per handle, by its max_atoms, so that a structure's sums do not depend on what
+ * shares its launch.  The picks are shared by the handles of the process and, with
+ * NEPX_TUNE_FILE set, kept in that file.  nepx_get_tuning reports the choices of
+ * the latest call and *tuned = 1 if they are kept.  nepx_set_tuning fixes
  * them for every later call on the handle (no timing runs), for example to
  * repeat a run's summation order bit for bit; values outside the lists
  * above return NEPX_ERR_ARG.  nepx_set_precision with a new mode lets the
