@@ -21,6 +21,7 @@ struct NeighborBuffers {
   int* nl_a = nullptr;   // [N][st_a], st_a = mn_a rounded up to eight
   int* heads = nullptr;  // [N][st_h] length and every eighth entry of the angular rows
   int st_a = 0, st_h = 0;
+  bool heads_after_filter = false;   // the heads' memory is the Verlet rows': not the filter's to write
   // the cooperative rebuild kernel: its grid-barrier counters (arrivals,
   // generation), per-block partial sums of the cell scan, its block count
   unsigned* gsync = nullptr;         // [2]

@@ -958,7 +958,7 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
       const int at = ca + __popc(ma & below);
       if (at < mn_a) {
         arow[at] = j;
-        if (at % 8 == 0) hrow[1 + at / 8] = j;
+        if (at % 8 == 0 && heads) hrow[1 + at / 8] = j;
         eout[at] = make_float4(x12, y12, z12, __int_as_float(t2 << kRowTypeShift));
       }
     }
@@ -983,7 +983,7 @@ k_filter_radial(const ModelParams p, int N, const Box* __restrict__ box,
   if (active && gl == 0) {
     nn_r[i] = min(cr, mn_r);
     nn_a[i] = min(ca, mn_a);
-    hrow[0] = min(ca, mn_a);
+    if (heads) hrow[0] = min(ca, mn_a);
     if (cr > mn_r) atomicOr(&st->overflow, 2);
     if (ca > mn_a) atomicOr(&st->overflow, 4);
     atomicMax(&st->max_nn[1], cr);
@@ -1678,6 +1678,22 @@ __device__ __forceinline__ void load8(const int* __restrict__ at, int (&v)[8])
       : "l"(at));
 }
 
+// The rows of heads from finished angular rows, a thread per slot (the filter
+// writes them on its way, except where they share the memory of its Verlet rows).
+__global__ void __launch_bounds__(256)
+k_row_heads(int N, const int* __restrict__ nn_a, const int* __restrict__ nl_a, int st_a,
+            int* __restrict__ heads, int st_h)
+{
+  const int slots = 1 + st_a / 8;
+  const long long k = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int i = static_cast<int>(k / slots), q = static_cast<int>(k % slots);
+  if (i >= N) return;
+  const int n = nn_a[i];
+  if (q == 0) heads[static_cast<size_t>(i) * st_h] = n;
+  else if (8 * (q - 1) < n)
+    heads[static_cast<size_t>(i) * st_h + q] = nl_a[static_cast<size_t>(i) * st_a + 8 * (q - 1)];
+}
+
 // Slot of atom i in an ascending row, -1 if it is not there (a truncated row):
 // the last block of eight whose head is not above i, from the row of heads (the
 // row's length, then its every eighth entry), then the place in that block.  Two
@@ -2039,7 +2055,8 @@ void launch_filter_tf(Engine& e, int N, cudaStream_t s)
     allow_smem(kernel, smem);
     kernel<<<blocks, kBlock, smem, s>>>(p, N, e.d_box, e.scratch.sites, e.d_nstate, nb.nn_v,
                                         nb.nl_v, nb.mn_v, nb.nn_r, nb.nl_r, nb.mn_r, nb.nn_a,
-                                        nb.nl_a, nb.mn_a, nb.st_a, nb.heads, nb.st_h,
+                                        nb.nl_a, nb.mn_a, nb.st_a,
+                                        nb.heads_after_filter ? nullptr : nb.heads, nb.st_h,
                                         e.scratch.f12, e.scratch.qrad);
   };
   const int bin = filter_bin<KM>(p);
@@ -2346,7 +2363,15 @@ void launch_descriptor(Engine& e, int N, const double*, const int*, cudaStream_t
 {
   const bool small = small_shape(e.params);
   const bool high = high_degree(e.params);
-  if (!e.use_xr) launch_filter(e, N, stream);
+  if (!e.use_xr) {
+    launch_filter(e, N, stream);
+    if (e.nbr.heads_after_filter) {
+      const NeighborBuffers& nb = e.nbr;
+      const long long slots = static_cast<long long>(N) * (1 + nb.st_a / 8);
+      k_row_heads<<<static_cast<unsigned>((slots + 255) / 256), 256, 0, stream>>>(
+        N, nb.nn_a, nb.nl_a, nb.st_a, nb.heads, nb.st_h);
+    }
+  }
   if (high) launch_fused_g<kHighFusedGroup, kMaxN, kMaxBasis, kMaxN, 8, 2>(e, N, stream);
   else if (e.group == 32 && fused_wide_groups(e)) launch_fused_wide<32>(e, N, stream);
   else if (e.group == 16 && fused_wide_groups(e)) launch_fused_wide<16>(e, N, stream);

@@ -72,51 +72,55 @@ struct Carver {
   }
 };
 
-// Bytes of alpha, rounded up, and of it and the site energies.
-size_t alpha_bytes(const nepx::Engine& e, size_t N)
+// A call's buffers from `base` (nullptr: their size alone), for N atoms of e's
+// model; returns the bytes they take.  What only the neighbour update and the filter
+// read shares its memory with what is written after the filter: the head rows then
+// follow from the angular rows (heads_after_filter), the descriptor kernel writes
+// the rest, and the next call builds its rows anew.  So the rows of heads, which
+// grow with MN_angular, take no atom from what the array holds.
+size_t lay_out(const nepx::Engine& e, size_t N, unsigned char* base, nepx::Box*& d_box,
+               nepx::NeighborState*& d_nstate, nepx::NeighborBuffers& nb, nepx::ForceScratch& sc)
 {
-  return (sizeof(float) * N * e.params.T * nepx::alpha_stride(e.params) + 255) & ~size_t(255);
-}
-
-// Alpha and the site energies lie over the Verlet rows where these are large
-// enough: every call builds the rows anew, and the filter has read them before
-// the descriptor kernel writes either.
-bool over_verlet_rows(const nepx::Engine& e, size_t N)
-{
-  return alpha_bytes(e, N) + sizeof(double) * N <= sizeof(int) * N * e.nbr.mn_v;
+  const nepx::ModelParams& p = e.params;
+  const size_t cells = std::max<size_t>(N, 4096);
+  Carver c{base};
+  d_box = c.take<nepx::Box>(1);
+  d_nstate = c.take<nepx::NeighborState>(1);
+  nb.nn_r = c.take<int>(N);
+  nb.nl_r = c.take<int>(N * nb.mn_r);
+  nb.nn_a = c.take<int>(N);
+  nb.nl_a = c.take<int>(N * nb.st_a);
+  nb.gsync = c.take<unsigned>(2);
+  nb.scan_part = c.take<int>(nb.rebuild_blocks);
+  nb.gsync_dirty = false;
+  sc.sites = c.take<nepx::Site>(N);
+  sc.qrad = c.take<float>(N * p.nR);
+  sc.f12 = c.take<float4>(N * std::max(nb.mn_a, 2));
+  nb.cell_sites = reinterpret_cast<nepx::Site*>(sc.f12);   // as engine_create has it
+  Carver early = c, late = c;
+  nb.nn_v = early.take<int>(N);
+  nb.nl_v = early.take<int>(N * nb.mn_v);
+  nb.cell_count = early.take<int>(cells);
+  nb.cell_start = early.take<int>(cells);
+  nb.cell_atoms = early.take<int>(N);
+  nb.cell_of = early.take<int>(N);
+  nb.x0 = early.take<double>(3 * N);
+  nb.cell_cap = static_cast<int>(cells);
+  nb.heads = late.take<int>(N * nb.st_h);
+  nb.heads_after_filter = true;
+  sc.alpha = late.take<float>(N * p.T * nepx::alpha_stride(p));
+  sc.pe_ann = late.take<double>(N);
+  sc.acoef = late.take<float>(N * p.nA * p.nlm);
+  return std::max(early.used, late.used);
 }
 
 size_t bytes_needed(const nepx::Engine& e, int n)
 {
-  Carver c{nullptr};
-  const nepx::NeighborBuffers& nb = e.nbr;
-  const size_t N = n;
-  const size_t cells = std::max<size_t>(N, 4096);
-  c.take<nepx::Box>(1);
-  c.take<nepx::NeighborState>(1);
-  c.take<int>(N);               // nn_v
-  c.take<int>(N * nb.mn_v);     // nl_v
-  c.take<int>(N);               // nn_r
-  c.take<int>(N * nb.mn_r);     // nl_r
-  c.take<int>(N);               // nn_a
-  c.take<int>(N * nb.st_a);     // nl_a
-  c.take<int>(N * nb.st_h);     // heads
-  c.take<unsigned>(2);                   // grid-barrier counters
-  c.take<int>(nb.rebuild_blocks);        // cell-scan partial sums
-  c.take<int>(cells);           // cell_count
-  c.take<int>(cells);           // cell_start
-  c.take<int>(N);               // cell_atoms
-  c.take<int>(N);               // cell_of
-  c.take<double>(3 * N);        // x0
-  c.take<nepx::Site>(N);
-  c.take<float>(N * e.params.nR);
-  c.take<float4>(N * std::max(nb.mn_a, 2));
-  if (!over_verlet_rows(e, N)) {
-    c.take<unsigned char>(alpha_bytes(e, N));
-    c.take<double>(N);
-  }
-  c.take<float>(N * e.params.nA * e.params.nlm);
-  return c.used;
+  nepx::Box* box = nullptr;
+  nepx::NeighborState* state = nullptr;
+  nepx::NeighborBuffers nb = e.nbr;
+  nepx::ForceScratch sc;
+  return lay_out(e, n, nullptr, box, state, nb, sc);
 }
 
 // The handle's engine runs the launches with its per-call buffers pointed
@@ -198,39 +202,7 @@ extern "C" int nepx_compute_noalloc(nepx_t* h, const nepx_box* box, int n, const
   auto s = static_cast<cudaStream_t>(stream);
   {
     BorrowedBuffers keep(e);
-    Carver c{static_cast<unsigned char*>(base)};
-    const size_t N = n;
-    const size_t cells = std::max<size_t>(N, 4096);
-    nepx::NeighborBuffers& nb = e.nbr;
-    e.d_box = c.take<nepx::Box>(1);
-    e.d_nstate = c.take<nepx::NeighborState>(1);
-    nb.nn_v = c.take<int>(N);
-    nb.nl_v = c.take<int>(N * nb.mn_v);
-    nb.nn_r = c.take<int>(N);
-    nb.nl_r = c.take<int>(N * nb.mn_r);
-    nb.nn_a = c.take<int>(N);
-    nb.nl_a = c.take<int>(N * nb.st_a);
-    nb.heads = c.take<int>(N * nb.st_h);
-    nb.gsync = c.take<unsigned>(2);
-    nb.scan_part = c.take<int>(nb.rebuild_blocks);
-    nb.gsync_dirty = false;
-    nb.cell_count = c.take<int>(cells);
-    nb.cell_start = c.take<int>(cells);
-    nb.cell_atoms = c.take<int>(N);
-    nb.cell_of = c.take<int>(N);
-    nb.x0 = c.take<double>(3 * N);
-    nb.cell_cap = static_cast<int>(cells);
-    e.scratch.sites = c.take<nepx::Site>(N);
-    e.scratch.qrad = c.take<float>(N * e.params.nR);
-    e.scratch.f12 = c.take<float4>(N * std::max(nb.mn_a, 2));
-    nb.cell_sites = reinterpret_cast<nepx::Site*>(e.scratch.f12);   // as engine_create has it
-    unsigned char* spent = over_verlet_rows(e, N) ? reinterpret_cast<unsigned char*>(nb.nl_v)
-                                                  : c.take<unsigned char>(alpha_bytes(e, N));
-    e.scratch.alpha = reinterpret_cast<float*>(spent);
-    e.scratch.pe_ann = over_verlet_rows(e, N)
-                         ? reinterpret_cast<double*>(spent + alpha_bytes(e, N))
-                         : c.take<double>(N);
-    e.scratch.acoef = c.take<float>(N * e.params.nA * e.params.nlm);
+    lay_out(e, n, static_cast<unsigned char*>(base), e.d_box, e.d_nstate, e.nbr, e.scratch);
     e.capacity = n;
     e.precision = 0;     // FP32 ANN: the mixed path's buffers are not in the static array
     e.use_xr = false;
@@ -238,7 +210,7 @@ extern "C" int nepx_compute_noalloc(nepx_t* h, const nepx_box* box, int n, const
     nepx::engine_choose(e, n, d_pos, d_type, s, nepx::ChoiceScope::kByCall, false);
     // the array keeps the previous call's contents: clear the flags, rebuild
     cudaMemsetAsync(e.d_nstate, 0, sizeof(nepx::NeighborState), s);
-    cudaMemsetAsync(nb.gsync, 0, 2 * sizeof(unsigned), s);
+    cudaMemsetAsync(e.nbr.gsync, 0, 2 * sizeof(unsigned), s);
     nepx::launch_set_box(e, b, s);
     nepx::launch_neighbor_update(e, n, d_pos, d_type, true, s);
     nepx::launch_force(e, n, d_pos, d_type, d_pe, d_force, d_virial, false, s);
