@@ -1997,6 +1997,14 @@ bool exact_shape(const ModelParams& p)
   return p.nR == kSmallN && p.nA == kSmallN && p.kR == kSmallK && p.kA == kSmallK && p.L_max == 4;
 }
 
+// Builds of the exact shape: everywhere the model has it, except at four CTAs per SM
+// with the angular force inside. At 128 registers the straight-line form spills 192
+// bytes there, the general one of the same bounds none (force call of 24,000 water
+// atoms in that build: 196 -> 182 us at 4 lanes, 182 -> 173 at 8; the three-CTA
+// build takes 171).
+template <int KM, int LMAX, int MINB, bool FF>
+constexpr bool exact_build() { return KM == kSmallK && LMAX == 4 && !(MINB == 4 && FF); }
+
 template <int G, int NRM, int KM, int NAM, bool XR, int LMAX, int MINB, bool TC, bool FF, bool EX>
 void launch_fused_tx(Engine& e, int N, cudaStream_t s)
 {
@@ -2018,7 +2026,7 @@ void launch_fused_tx(Engine& e, int N, cudaStream_t s)
 template <int G, int NRM, int KM, int NAM, bool XR, int LMAX, int MINB, bool TC, bool FF = false>
 void launch_fused_t(Engine& e, int N, cudaStream_t s)
 {
-  if constexpr (KM == kSmallK && LMAX == 4) {
+  if constexpr (exact_build<KM, LMAX, MINB, FF>()) {
     if (exact_shape(e.params)) {
       launch_fused_tx<G, NRM, KM, NAM, XR, LMAX, MINB, TC, FF, true>(e, N, s);
       return;
@@ -2122,7 +2130,8 @@ void set_fused_smem_t(const ModelParams& p)
     if (exact_shape(p)) {
       allow_smem(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, false, true>, bytes);
       allow_smem(k_nep_fused<G, NRM, KM, NAM, true, LMAX, MINB, TC, false, true>, bytes);
-      allow_smem(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, true, true>, bytes);
+      allow_smem(k_nep_fused<G, NRM, KM, NAM, false, LMAX, MINB, TC, true,
+                             exact_build<KM, LMAX, MINB, true>()>, bytes);
       return;
     }
   }
