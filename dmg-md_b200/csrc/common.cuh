@@ -158,20 +158,6 @@ struct MinImage {
   }
 };
 
-// Displacement r_j - r_i: the double difference rounded to float, then the
-// float minimum image -- the operand order of the reference's filter
-// (nep.cu:542-549), so neighbour predicates agree bit for bit.
-__device__ __forceinline__ void displacement(const Box& b, const double* __restrict__ x,
-                                             const double* __restrict__ y,
-                                             const double* __restrict__ z, double xi, double yi,
-                                             double zi, int j, float& dx, float& dy, float& dz)
-{
-  dx = __ldg(x + j) - xi;
-  dy = __ldg(y + j) - yi;
-  dz = __ldg(z + j) - zi;
-  mic_f32(b, dx, dy, dz);
-}
-
 // One atom as the neighbour sweeps read it: position and type in one
 // 32-byte record (one sector), repacked from the SoA inputs at every force
 // call.  The SoA layout would touch four cache lines per neighbour.
@@ -201,8 +187,9 @@ __device__ __forceinline__ void site_load_coherent(const Site* sites, int j, dou
                : "memory");
 }
 
-// Displacement from (xi, yi, zi) to a loaded site and the site's type, same
-// arithmetic as displacement().
+// Displacement from (xi, yi, zi) to a loaded site, and the site's type: the double
+// difference rounded to float, then the float minimum image -- the operand order of
+// the reference's filter (nep.cu:542-549), so neighbour predicates agree bit for bit.
 __device__ __forceinline__ void site_delta(const Box& b, const double2& a, const double2& c,
                                            double xi, double yi, double zi, float& dx, float& dy,
                                            float& dz, int& tj)
@@ -223,16 +210,6 @@ __device__ __forceinline__ void site_delta(const MinImage& mic, const double2& a
   dz = c.x - zi;
   tj = static_cast<int>(__double_as_longlong(c.y));
   mic(dx, dy, dz);
-}
-
-// Displacement to site j and j's type.
-__device__ __forceinline__ void site_displacement(const Box& b, const Site* __restrict__ sites,
-                                                  double xi, double yi, double zi, int j,
-                                                  float& dx, float& dy, float& dz, int& tj)
-{
-  double2 a, c;
-  site_load(sites, j, a, c);
-  site_delta(b, a, c, xi, yi, zi, dx, dy, dz, tj);
 }
 
 // Skin criterion of atom i at its new position (reference

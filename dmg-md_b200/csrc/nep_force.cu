@@ -2258,21 +2258,32 @@ void launch_fused_wide(Engine& e, int N, cudaStream_t s)
 }
 
 template <int G, int KM, int NAM, int LMAX>
+void launch_gather_xr(Engine& e, int N, double* pe, double* force, double* virial,
+                      bool accumulate, cudaStream_t s)
+{
+  // a single system takes the images' scheme whatever its box
+  if (e.xr.from_box || (e.xr.kinds & kSmallRows))
+    launch_gather_t<G, KM, NAM, kImages, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
+  if (e.xr.from_box || !(e.xr.kinds & kLargeRows)) return;
+  launch_gather_t<G, KM, NAM, kLarge, LMAX, LMAX == 4 ? 4 : 0>(e, N, pe, force, virial, accumulate,
+                                                                s);
+}
+
+template <int G, int KM, int NAM, int LMAX>
 void launch_gather_g(Engine& e, int N, double* pe, double* force, double* virial,
                      bool accumulate, cudaStream_t s)
 {
   if (e.use_xr) {
-    // a single system takes the images' scheme whatever its box
-    if (e.xr.from_box || (e.xr.kinds & kSmallRows))
-      launch_gather_t<G, KM, NAM, kImages, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
-    if (e.xr.from_box || !(e.xr.kinds & kLargeRows)) return;
-    if (LMAX == 4) launch_gather_t<G, KM, NAM, kLarge, LMAX, 4>(e, N, pe, force, virial, accumulate, s);
-    else launch_gather_t<G, KM, NAM, kLarge, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
-  } else if (LMAX == 4 && e.gather_minb == 4) {
-    launch_gather_t<G, KM, NAM, kVerlet, LMAX, 4>(e, N, pe, force, virial, accumulate, s);
-  } else {
-    launch_gather_t<G, KM, NAM, kVerlet, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
+    launch_gather_xr<G, KM, NAM, LMAX>(e, N, pe, force, virial, accumulate, s);
+    return;
   }
+  if constexpr (LMAX == 4) {
+    if (e.gather_minb == 4) {
+      launch_gather_t<G, KM, NAM, kVerlet, LMAX, 4>(e, N, pe, force, virial, accumulate, s);
+      return;
+    }
+  }
+  launch_gather_t<G, KM, NAM, kVerlet, LMAX, 0>(e, N, pe, force, virial, accumulate, s);
 }
 
 }  // namespace
@@ -2413,8 +2424,8 @@ void launch_gather(Engine& e, int N, const double*, const int*, double* pe, doub
     launch_gather_g<kHighGroup, kMaxBasis, kMaxN, 8>(e, N, pe, force, virial, accumulate, stream);
   else if (small && e.gather_group == 32)
     launch_gather_g<32, kSmallK, kSmallN, 4>(e, N, pe, force, virial, accumulate, stream);
-  else if (small && e.gather_group == 16)
-    launch_gather_g<16, kSmallK, kSmallN, 4>(e, N, pe, force, virial, accumulate, stream);
+  else if (small && e.gather_group == 16 && e.use_xr)   // (no choice takes 16 on Verlet rows)
+    launch_gather_xr<16, kSmallK, kSmallN, 4>(e, N, pe, force, virial, accumulate, stream);
   else if (e.gather_group == 4) {
     if (small) launch_gather_g<4, kSmallK, kSmallN, 4>(e, N, pe, force, virial, accumulate, stream);
     else launch_gather_g<4, kMaxBasis, kMaxN, 4>(e, N, pe, force, virial, accumulate, stream);
