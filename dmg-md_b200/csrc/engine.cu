@@ -320,7 +320,11 @@ LaunchChoices& choices(Engine& e) { return e; }
 //                       8,000: 35 25 29 26
 // (1,551 water atoms in the descriptor kernel: 44 38 38 36.)  A rule also gives
 // every process of a small system the same sums; its lines are powers of two
-// because the picks are kept by size class.
+// because the picks are kept by size class.  It holds for what the table measured,
+// the usual shape in FP32; other shapes and the mixed modes are timed at every size,
+// and take it only where nothing may be timed.
+bool small_rule(const Engine& e) { return fused_wide_groups(e); }
+
 LaunchChoices small_choices(Engine& e, int N)
 {
   LaunchChoices c;
@@ -338,27 +342,28 @@ LaunchChoices small_choices(Engine& e, int N)
 }
 
 // A batch handle or server for many atoms whose first step holds few: nothing to
-// time on yet, and a small step's lanes would stay for the full ones.  Lanes that
-// serve both (ms; 48 requests, some 13,000 atoms a step, and one batch of 248,000
-// atoms; the gather at 4 8 16 32 lanes, then the descriptor kernel):
-//   descriptor kernel at 4:  29.9 25.9 24.7 24.0;  2.67 2.68 2.74 2.90
-//   gather at 16:            24.7 25.4 25.4 25.4;  2.74 2.86 3.34 4.08
-// (the gather of a small box evaluates both angular forces of an edge, so it gains
-// from more lanes for longer than the descriptor kernel).
-LaunchChoices filling_choices(const Engine& e)
+// time on yet, and a small step's lanes (up to 32 in the descriptor kernel) would
+// stay for the full ones.  Lanes that serve both (ms; lanes of the descriptor kernel
+// and the gather 4/8, 4/16, 4/32, 8/8, 8/16, 8/32, 16/32):
+//   stream of 1,324 atoms    4.26  3.90  3.77  4.02  3.83  3.69  3.70
+//   of 4,526                 5.94  5.44  5.13  5.55  4.87  4.59  4.56
+//   of 72,225               15.77 14.79 14.53 16.22 15.20 14.60 15.05
+//   one batch of 242,031     2.85  2.90  3.06  2.88  2.93  3.08  3.09   (FP32:
+//                            2.69  2.74  2.90  2.93  2.98  3.16  3.51; 32/32: 4.2)
+// A stream's steps hold mostly the segments that go on, so its gather gains from 32
+// lanes up to the largest; a batch that comes full from the start is timed.
+LaunchChoices filling_choices()
 {
   LaunchChoices c;
-  c.group = 4;
-  c.fused_minb = fused_wide_groups(e) ? 4 : 3;
-  c.f12_group = 8;
-  c.gather_group = 16;
+  c.group = c.f12_group = 8;
+  c.gather_group = 32;
   return c;
 }
 
-// The launch variants timed on the given system, the fastest left in e; the
-// 32-lane gather only for wide_gather.
+// The launch variants timed on the given system, the fastest left in e: groups of 16
+// and 32 lanes in size band 0, the 32-lane gather in bands 0 and 1.
 void time_variants(Engine& e, int N, const double* pos, const int* type, cudaStream_t stream,
-                   bool wide_gather)
+                   int band)
 {
   const int groups[2] = {4, 8};   // candidate lanes per center
   cudaEvent_t a, b;
@@ -382,7 +387,8 @@ void time_variants(Engine& e, int N, const double* pos, const int* type, cudaStr
   if (!e.use_xr) {
     float best = 1e30f;
     int pick = e.filter_group;
-    for (int g : groups) {
+    const int last = band == 0 && wide_groups(e.params) ? 32 : 8;
+    for (int g = 4; g <= last; g *= 2) {
       e.filter_group = g;
       const float t = median(5, [&] { launch_filter(e, N, stream); });
       if (t < best) {
@@ -430,7 +436,7 @@ void time_variants(Engine& e, int N, const double* pos, const int* type, cudaStr
   int pick_g = 8, pick_gm = 3;
   const int gm_last = !e.use_xr && e.params.L_max <= 4 ? 4 : 3;
   const int gather_lanes[3] = {4, 8, 32};
-  const int n_lanes = wide_gather ? 3 : 2;
+  const int n_lanes = band <= 1 && wide_groups(e.params) ? 3 : 2;
   for (int gm = 3; gm <= gm_last; ++gm)
     for (int k = 0; k < n_lanes; ++k) {
       e.gather_minb = gm;
@@ -482,8 +488,10 @@ void engine_choose(Engine& e, int N, const double* pos, const int* type, cudaStr
 {
   if (e.pinned) return;
   const bool by_handle = scope == ChoiceScope::kByHandle;
-  // the size that sets the choice: the call's, or the largest the handle serves
-  const int n = by_handle ? e.capacity : N;
+  // the size that sets the choice: the call's, or for a small handle's one set the
+  // largest it serves
+  const bool filling = by_handle && N < kWideAtoms && e.capacity >= kWideAtoms;
+  const int n = by_handle && N < kWideAtoms ? e.capacity : N;
   const Engine::ChosenFor want{scope, by_handle ? -1 : size_class(n), e.use_xr};
   if (e.tuned && e.chosen_for == want) return;
   const int band = n < kWideAtoms ? 0 : n < kGatherWideAtoms ? 1 : 2, path = e.use_xr ? 1 : 0;
@@ -492,23 +500,25 @@ void engine_choose(Engine& e, int N, const double* pos, const int* type, cudaStr
   bool fixed = true;
   if (by_handle && e.has_by_handle) {
     choices(e) = e.by_handle;
+  } else if (filling) {
+    choices(e) = filling_choices();
   } else if (tune_lookup(key, known, may_time)) {
     choices(e) = known;
-  } else if (band == 0) {
+  } else if (band == 0 && small_rule(e)) {
     choices(e) = small_choices(e, n);
     if (may_time) tune_store(key, choices(e));
-  } else if (by_handle && N < kWideAtoms) {
-    choices(e) = filling_choices(e);
   } else if (!by_handle && e.has_timed[path][band]) {
     choices(e) = e.timed[path][band];
   } else if (may_time && can_time(stream)) {
-    time_variants(e, N, pos, type, stream, band == 1);
+    time_variants(e, N, pos, type, stream, band);
     e.timed[path][band] = e;
     e.has_timed[path][band] = true;
     tune_store(key, choices(e));
   } else {
     const int other = band == 1 ? 2 : 1;
-    choices(e) = e.has_timed[path][other] ? e.timed[path][other] : LaunchChoices{};
+    choices(e) = band == 0                 ? small_choices(e, n)
+                 : e.has_timed[path][other] ? e.timed[path][other]
+                                            : LaunchChoices{};
     fixed = false;
   }
   e.tuned = fixed;

@@ -171,8 +171,8 @@ size_t fused_tc_smem_bytes(const ModelParams& p);
 // Lane groups per center that kernels are built for; 16 and 32 run as 8 where
 // a kernel has no build for the model.
 inline bool lanes_built(int g) { return g == 4 || g == 8 || g == 16 || g == 32; }
-// Systems below this many atoms take their lanes from a rule on the size
-// (engine_choose); from there on the chip is full at 4 or 8 lanes.
+// Systems below this many atoms take up to 32 lanes per center (engine_choose);
+// from there on the chip is full at 4 or 8 lanes.
 constexpr int kWideAtoms = 4096;
 // Below this many the gather's 32-lane groups are timed too (8,000 carbon atoms,
 // lanes 4 8 32: 35 25 23 us).
@@ -191,8 +191,9 @@ bool wide_groups(const ModelParams& p);
 void set_fused_smem_limits(const ModelParams& p);
 
 // Sets the launch choices of a call of N atoms: nothing to do while they are those
-// of its size class and row path, or pinned.  A small system (below kWideAtoms)
-// takes its lanes from its size; otherwise each kernel variant is timed on the
+// of its size class and row path, or pinned.  A small system (below kWideAtoms) of
+// the usual shape in FP32 takes its lanes from its size; otherwise each kernel
+// variant is timed on the
 // given system (a few calls each, stream synchronised) and the fastest kept: the
 // lane-group size of the filter, descriptor, angular-force and gather kernels,
 // the CTAs per SM of the descriptor kernel and of the gather, and whether the

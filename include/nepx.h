@@ -332,10 +332,11 @@ int nepx_set_precision(nepx_t* handle, int mode);
  *       (three CTAs of 256 per SM), 4 = held to four CTAs (64 registers, a
  *       third more warps)
  * 16 and 32 lanes run as 8 where a kernel has no build of them for the model.
- * They follow the size of each call: below 4,096 atoms they are set by it, from
- * there on a handle's first call of a size times the variants and keeps the
- * fastest (the autotuner; once per row path below and above 16,384 atoms; not
- * under stream capture).  Batches, servers and an md on explicit rows keep one set
+ * They follow the size of each call: below 4,096 atoms it sets them for models of
+ * the usual shape (n_max 4 4, basis 8 8, l_max 4) in FP32; otherwise a handle's
+ * first call of a size times the variants and keeps the fastest (the autotuner;
+ * once per row path below 4,096, below 16,384 and from there on; not under
+ * stream capture).  Batches, servers and an md on explicit rows keep one set
  * per handle, by its max_atoms, so that a structure's sums do not depend on what
  * shares its launch.  The picks are shared by the handles of the process and, with
  * NEPX_TUNE_FILE set, kept in that file.  nepx_get_tuning reports the choices of

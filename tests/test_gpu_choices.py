@@ -3,14 +3,18 @@ a handle that serves a small system and then a large one takes the large one's
 lanes for it, and the small one's again afterwards, in direct calls and in an MD
 between whose runs the handle served another size.  A batch handle and a server
 keep one set for their life (a structure's sums must not depend on what shares
-its launch), which is not that of a small first step.  Pinned choices stay, and a
+its launch), whose descriptor lanes are not those of a small first step.  Pinned choices stay, and a
 call under stream capture times nothing."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import oracle
 import workloads
-from conftest import potential
+from conftest import ROOT, potential
 from test_gpu_force import assert_close
 
 torch = pytest.importorskip("torch")
@@ -83,7 +87,7 @@ def test_server_whose_first_step_is_small():
     srv = nepx.Server(pot, max_atoms=18000, max_struct=8)
     got = [srv.wait(srv.submit(structs[0][0], structs[0][2], structs[0][1]))]
     choices = pot.tuning()
-    assert choices[0]["fused_group"] <= 8 and choices[0]["gather_group"] <= 16
+    assert choices[0]["fused_group"] == 8             # not the 32 of 60 atoms
     tickets = [srv.submit(t, p, h) for t, h, p in structs]
     got += [srv.wait(k) for k in tickets]
     assert pot.tuning() == choices
@@ -124,3 +128,37 @@ def test_nothing_is_timed_under_capture():
                  "captured call")
     del graph
     pot.close()
+
+
+SCRIPT = r"""
+import sys
+sys.path.insert(0, %r); sys.path.insert(0, %r)
+import numpy as np, torch, workloads, nepx, os, tempfile
+from conftest import potential
+t, h, p = workloads.water(n_mol=300, seed=11)
+wide = workloads.write_nep(os.path.join(tempfile.mkdtemp(), "nep.txt"), symbols=("O", "H"),
+                           rc=(5.0, 4.0), mn=(200, 100), n_max=(6, 5), basis=(12, 10), seed=3,
+                           q_scaler=0.05)
+tt = torch.as_tensor(t, device="cuda"); pp = torch.as_tensor(p, device="cuda")
+for path, mode in ((potential("nep_water.txt"), "fp32"), (potential("nep_water.txt"), "mixed"),
+                   (wide, "fp32")):
+    pot = nepx.Potential(path, max_atoms=len(t))
+    pot.set_precision(mode)
+    sys.stderr.write("handle\n"); sys.stderr.flush()
+    pot.compute(tt, h, pp, sync_check=True)
+    assert pot.tuning()[1]
+    pot.close()
+"""
+
+
+def test_small_systems_outside_the_rule_are_timed():
+    """The rule by size was measured for the usual shape in FP32; a mixed mode and
+    another shape below its line are timed (NEPX_VERBOSE names each timing)."""
+    code = SCRIPT % (os.path.join(ROOT, "dmg-md_b200"), os.path.join(ROOT, "tests"))
+    env = {k: v for k, v in os.environ.items() if k != "NEPX_TUNE_FILE"}
+    r = subprocess.run([sys.executable, "-c", code], env=dict(env, NEPX_VERBOSE="1"), cwd=ROOT,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    usual, mixed, other = r.stderr.split("handle\n")[1:]
+    assert "autotune" not in usual
+    assert "autotune (N=900)" in mixed and "autotune (N=900)" in other
