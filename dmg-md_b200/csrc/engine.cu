@@ -249,8 +249,10 @@ int size_class(int N)
 TuneKey tune_key(const Engine& e, int N)
 {
   const ModelParams& p = e.params;
+  // the last field: what the picks mean (raised when a value comes to name another
+  // build or form, so that a file of the library before is not read as this one's)
   TuneKey k{{e.device, e.use_xr ? 1 : 0, e.precision, p.T, p.nR, p.nA, p.kR, p.kA, p.L_max,
-             p.dim, p.H, p.num_inv, size_class(N), 3}};
+             p.dim, p.H, p.num_inv, size_class(N), 4}};
   return k;
 }
 

@@ -106,11 +106,14 @@ def test_server_whose_first_step_is_small():
     pot.close()
 
 
-def test_nothing_is_timed_under_capture():
+def test_nothing_is_timed_under_capture(tmp_path):
     import nepx
+    # a model of its own: no other test of this process has timed it
+    path = workloads.write_nep(str(tmp_path / "nep.txt"), symbols=("O", "H"), rc=(6.0, 4.0),
+                               mn=(250, 100), H=17, seed=12, q_scaler=0.02)
     ts, hs, ps = workloads.water(n_mol=250, seed=9)
     tl, hl, pl = workloads.water(n_mol=1700, seed=10)           # 5,100 atoms: timed
-    pot = nepx.Potential(PATH, max_atoms=len(tl))
+    pot = nepx.Potential(path, max_atoms=len(tl))
     dev = _device(ts, ps)
     pot.compute(dev[0], hs, dev[1], sync_check=True)
     dev = _device(tl, pl)
@@ -124,7 +127,7 @@ def test_nothing_is_timed_under_capture():
     assert pot.tuning()[1] is False and _narrow(pot)
     graph.replay()
     torch.cuda.synchronize()
-    assert_close(oracle.OracleModel(PATH).compute(tl, hl, pl), [x.cpu().numpy() for x in out],
+    assert_close(oracle.OracleModel(path).compute(tl, hl, pl), [x.cpu().numpy() for x in out],
                  "captured call")
     del graph
     pot.close()
