@@ -248,14 +248,15 @@ int grid(int n) { return (n + kThreads - 1) / kThreads; }
 }  // namespace
 
 // Device bytes one served atom occupies: the handle's per-atom buffers of the
-// explicit-row path (radial and angular rows, angular partial forces, site
-// records, cell slots, descriptor scratch) and the server's two arena
-// buffers and I/O blocks.
+// explicit-row path (radial and angular rows, the angular rows' indices and heads,
+// angular partial forces, site records, cell slots, descriptor scratch) and the
+// server's two arena buffers and I/O blocks.
 size_t served_bytes_per_atom(const Engine& e)
 {
   const NeighborBuffers& nb = e.nbr;
   const ModelParams& p = e.params;
   size_t b = 16 * static_cast<size_t>(nb.mn_r + nb.mn_a);   // explicit rows (float4)
+  b += sizeof(int) * static_cast<size_t>(nb.st_a + nb.st_h);  // angular indices and heads
   b += 16 * static_cast<size_t>(nb.mn_a);                    // angular partial forces
   b += 2 * sizeof(int) + sizeof(Site) + 1 + 2 * sizeof(int); // counts, sites, flag, cell slots
   b += sizeof(float) * (static_cast<size_t>(p.nA) * p.nlm + p.T * alpha_stride(p) + p.nR);

@@ -169,6 +169,21 @@ def test_server_admits_by_device_memory():
     srv.close()
 
 
+def test_served_bytes_count_the_index_rows(tmp_path):
+    """80 more angular slots cost a served atom the edge and the force of each (16
+    bytes), its index (4), and eight more words of heads."""
+    import nepx
+    per_atom = []
+    for mn_a in (64, 128):               # 80 and 160 slots
+        path = workloads.write_nep(str(tmp_path / ("nep%d.txt" % mn_a)), mn=(160, mn_a), seed=2)
+        pot = nepx.Potential(path, max_atoms=64)
+        srv = nepx.Server(pot, max_atoms=64, max_struct=2)
+        per_atom.append(srv.memory()["bytes_per_atom"])
+        srv.close()
+        pot.close()
+    assert per_atom[1] - per_atom[0] == 80 * (16 + 16 + 4) + 8 * 4
+
+
 def _md_stream(seed):
     """MD segments of water in small, large and slab boxes (300 K, 1 fs:
     the hydrogens pass skin / 2 within a few tens of steps) mixed with single
