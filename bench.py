@@ -81,12 +81,12 @@ K_B = 8.617343e-5
 # per SM: the builds the autotuner picks for this model), dram__bytes_read.sum
 # + dram__bytes_write.sum of one ncu-captured launch each on the large-carbon
 # system at 1,000,000 atoms (--ncell 50), divided by its atoms (traffic grows
-# with the atoms processed).  An earlier build's capture: the present kernels
-# move 4.66 kB per atom (the filter also writes the angular edges).  Keyed by
-# workload and the kernel list; another form reports no traffic.
+# with the atoms processed): read + written by the filter, the descriptor kernel
+# and the gather.  Keyed by workload and the kernel list; another form reports no
+# traffic.
 TRAFFIC_PER_ATOM = {
     ("carbon8m", ("k_filter_radial", "k_nep_fused", "k_gather")):
-        (701.6 + 412.2 + 349.1 + 567.1 + 1359.3 + 292.3) * 1e6 / 1.0e6}
+        (811.4 + 1062.0 + 713.5 + 566.2 + 1409.7 + 99.1) * 1e6 / 1.0e6}
 FP32_LANES = 148 * 128          # B200: SMs x FP32 lanes
 SM_MAX_MHZ = 1965.0
 L2_NOTE = "flushed by a 512 MiB write before every %d-step chunk"

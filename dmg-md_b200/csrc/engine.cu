@@ -400,11 +400,10 @@ void time_variants(Engine& e, int N, const double* pos, const int* type, cudaStr
     }
     e.filter_group = pick;
   }
-  // the descriptor kernel's lanes per center, its occupancy builds (CTAs per
-  // SM) where the shape has two (the FP32 build of the small shape; the
-  // tensor-core build comes at 3), and the angular partial
-  // forces inside it (small shape, Verlet rows) or in their own kernel, whose
-  // lanes per center vary too
+  // the descriptor kernel's lanes per center, its two occupancy builds (CTAs per
+  // SM; degrees <= 4 in FP32, the tensor-core build has one), and the angular
+  // partial forces inside it (degrees <= 4, Verlet rows) or in their own kernel,
+  // whose lanes per center vary too
   const int n_minb = (fused_occupancy_variants(e.params) && e.precision == 0) ? 2 : 1;
   e.fuse_f12 = true;
   const int n_ff = fused_angular_force(e) ? 2 : 1;

@@ -180,8 +180,8 @@ constexpr int kGatherWideAtoms = 16384;
 // True when the descriptor kernel has 16- and 32-lane groups for this model
 // and precision.
 bool fused_wide_groups(const Engine& e);
-// True when the descriptor kernel comes in two occupancy builds (3 or 4 CTAs
-// per SM, Engine::fused_minb) for this model's shape.
+// True when the descriptor kernel comes in two occupancy builds (Engine::fused_minb
+// 3 or 4: as many CTAs per SM for the small shape, 2 or 3 for the general one).
 bool fused_occupancy_variants(const ModelParams& p);
 // True when the descriptor kernel writes the angular partial forces itself
 // (Engine::fuse_f12, degrees <= 4, on Verlet rows): no k_angular_f12.

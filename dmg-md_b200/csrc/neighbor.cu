@@ -16,9 +16,9 @@
 // returns at once, and never waits on the host.  Rows are row-major (atom i owns the contiguous
 // slots [i*MN, i*MN + count)) so the warp that owns a center reads and writes
 // coalesced.  The cell list is a counting sort on a grid of cells at least
-// (rc + skin)/2 wide with a 5x5x5 stencil; each Verlet row is sorted in
-// shared memory, which makes every later sum over neighbours ordered and
-// bitwise reproducible.
+// (rc + skin)/2 wide with a 5x5x5 stencil; each Verlet row is sorted (in
+// registers, above 256 entries in shared memory), which makes every later sum over
+// neighbours ordered and bitwise reproducible.
 #include <algorithm>
 #include <climits>
 
@@ -32,7 +32,7 @@ namespace {
 // Sixteen warps, a center per warp in the row build: CTAs of four warps hold the
 // same number, but four times the arrivals at every barrier.
 constexpr int kRebuildThreads = 512;
-constexpr int kRebuildCtas = 3;                      // per SM (42 registers)
+constexpr int kRebuildCtas = 3;                      // per SM (40 registers, the most for three; 72 bytes spilled)
 constexpr int kRebuildWarps = kRebuildThreads / 32;
 constexpr long long kGridWaitCycles = 4000000000ll;  // ~2 s at the B200 clock
 
@@ -214,7 +214,7 @@ struct RebuildArgs {
 //   4. atoms into their cells (index and site record, in cell order);
 //   5. Verlet rows: one warp per center gathers every candidate of the 5x5x5
 //      stencil (its rows along x, trimmed to the cells in reach) with float
-//      d^2 < (rc + skin)^2, sorts the row (bitonic, in registers up to 128
+//      d^2 < (rc + skin)^2, sorts the row (bitonic, in registers up to 256
 //      entries) and writes it with the reference positions of the next skin
 //      check.
 // They run only when the rebuild flag is set; the flag is the same for every
@@ -408,7 +408,8 @@ size_t rebuild_smem(int pow2) { return sizeof(int) * kRebuildWarps * (pow2 + 1);
 }  // namespace
 
 // Blocks of the cooperative rebuild: as many as can be resident at once (the
-// launch fails rather than oversubscribe), at most 16 per SM.
+// launch fails rather than oversubscribe): three per SM, fewer for long rows' sort
+// buffers.
 int neighbor_rebuild_blocks(int pow2_v)
 {
   int dev = 0, sms = 0, per_sm = 0;
@@ -420,7 +421,7 @@ int neighbor_rebuild_blocks(int pow2_v)
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_neighbor_rebuild, kRebuildThreads,
                                                     rebuild_smem(pow2_v)) != cudaSuccess)
     return 0;
-  return sms * std::min(per_sm, 16);
+  return sms * per_sm;
 }
 
 void launch_neighbor_update(Engine& e, int N, const double* pos, const int* type, bool force,

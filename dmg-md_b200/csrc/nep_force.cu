@@ -1,9 +1,7 @@
 // nep_force.cu -- NEP energy, force and virial on sm_100a.
 //
 // Three kernels per force call (four where k_angular_f12 runs by itself), each
-// giving a group of G lanes to one center: as the autotuner in engine.cu
-// finds (4 or 8, small systems' gather also 32), by a rule on the size below
-// 4096 atoms (up to 32).  Every phase is local to the group, so no CTA-wide barrier
+// giving a group of G lanes to one center (4 to 32: engine_choose).  Every phase is local to the group, so no CTA-wide barrier
 // follows the set-up (except in the tensor-core ANN, whose MMAs span the
 // CTA's centers).
 //
@@ -2118,7 +2116,7 @@ void launch_f12_t(Engine& e, int N, cudaStream_t s)
   launch_f12_tf<G, KM, NAM, LMAX, false>(e, N, s);
 }
 
-// FFI: the build also comes with the fused angular force (small shape)
+// FFI: the build also comes with the fused angular force (degrees <= 4)
 template <int G, int NRM, int KM, int NAM, int LMAX, int MINB, bool TC, bool FFI = false>
 void set_fused_smem_t(const ModelParams& p)
 {

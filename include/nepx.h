@@ -311,9 +311,9 @@ int nepx_md_device_state(nepx_md_t* md, double** d_pos, double** d_vel, double**
  * the hardware approximations of 1/sqrt (edge lengths), 1/x and sine/cosine
  * (the cutoff function), 2 ulp or about 4e-7 absolute, in place of the
  * FP32 mode's functions, whose errors are no larger than those of the sqrtf,
- * division and sincospif that the reference calls.  NEPX_ERR_UNSUPPORTED for models with dim >
- * 128 or more than 256 hidden units.  No counterpart in the reference (its
- * ANN is FP32 only).
+ * division and sincospif that the reference calls.  NEPX_ERR_UNSUPPORTED for
+ * models with dim > 128 or more than 1,024 hidden units over all types.  No
+ * counterpart in the reference (its ANN is FP32 only).
  */
 int nepx_set_precision(nepx_t* handle, int mode);
 
